@@ -30,10 +30,12 @@ constexpr int kPiece = 64;
 struct Ckpt {
     float4 a;  // pos.xyz, dst.x
     float4 b;  // dst.yzw, iter (bits)
-    uint4 c;   // nsamples, nptr xyz
+    uint4 c;   // nsamples, nptr
 };
 
 struct CkptVisitor {
+    static constexpr int kGather = 8;
+    static constexpr bool kEverySample = false;
     Ckpt* out;
     int cap, count, last;
     int* status;
@@ -42,14 +44,15 @@ struct CkptVisitor {
             Ckpt c;
             c.a = make_float4(s.pos.x, s.pos.y, s.pos.z, s.dst.x);
             c.b = make_float4(s.dst.y, s.dst.z, s.dst.w, __int_as_float(s.iter));
-            c.c = make_uint4((uint32_t)s.nsamples, s.nptr_x, s.nptr_y, s.nptr_z);
+            c.c = make_uint4((uint32_t)s.nsamples, s.nptr, 0u, 0u);
             out[count++] = c;
             last = s.nsamples;
         }
         return true;
     }
     __device__ __forceinline__ bool sample(int, const float4&, F3, float, int) { return true; }
-    __device__ __forceinline__ void segment_end(const RayState&, bool, bool) {}
+    template <bool UNIT>
+    __device__ __forceinline__ void segment_end(const RaycastParams&, const RayState&) {}
     __device__ __forceinline__ void fail(int code) { set_status(status, code); }
 };
 
@@ -58,6 +61,8 @@ struct CkptVisitor {
 // the sample's alpha, r = dot(dL/dc.rgb, src.rgb) (dL/dc.rgb is constant
 // along the ray) and the brick position.  24 bytes a sample.
 struct ReplayVisitor {
+    static constexpr int kGather = 32;  // without masks to skip by, a march is long: 31.0 ms a fit step, 31.5 at 16
+    static constexpr bool kEverySample = true;  // the gradient scatters empty samples too
     int first, last, n;
     float gx, gy, gz;  // dL/dc.rgb
     float T[kPiece];
@@ -76,7 +81,8 @@ struct ReplayVisitor {
         }
         return index + 1 < last;
     }
-    __device__ __forceinline__ void segment_end(const RayState&, bool, bool) {}
+    template <bool UNIT>
+    __device__ __forceinline__ void segment_end(const RaycastParams&, const RayState&) {}
     __device__ __forceinline__ void fail(int) {}
 };
 
@@ -238,18 +244,15 @@ __device__ __forceinline__ void pixel_of_strided(int& px, int& py) {
 
 }  // namespace
 
-// 7 resident CTAs (28 warps) per SM, at most 72 registers per thread (no
-// spills): the occupancy that measured fastest for the plain ray cast
-template <int FMT>
-__global__ void __launch_bounds__(128, 7) forward_ckpt_kernel(const __grid_constant__ RaycastParams p, int2* hdr,
-                                                           Ckpt* ckpt, int per_ray) {
-    int px, py;
-    pixel_of(px, py);
+// One pixel of the checkpointing forward.
+template <int FMT, bool UNIT>
+__device__ __forceinline__ void forward_pixel(const RaycastParams& p, int px, int py, int2* hdr, Ckpt* ckpt,
+                                              int per_ray, const PathSlots& path) {
     const vv_uniforms& u = p.u;
-    if (px >= u.width || py >= u.height) return;
-    const size_t pix = (size_t)py * u.width + px;
+    const bool inside = px < u.width && py < u.height;
+    const size_t pix = inside ? (size_t)py * u.width + px : 0;
     bool ok = true;
-    const WalkConsts k = walk_consts(p, fetch_node<false>(p, 0, 0, 0, ok));
+    const WalkConsts k = walk_consts(p, UNIT ? __ldg(p.walk) : fetch_node<false>(p, 0, 0, 0, ok));
     CkptVisitor vis;
     vis.out = ckpt + pix * (size_t)per_ray;
     vis.cap = per_ray;
@@ -260,66 +263,88 @@ __global__ void __launch_bounds__(128, 7) forward_ckpt_kernel(const __grid_const
     s.dst = make_float4(0.f, 0.f, 0.f, 0.f);
     s.nsamples = 0;
     F3 pos;
-    __shared__ uint2 path_w[kPathLevels][128];
-    __shared__ uint32_t path_p[kPathLevels][128];
-    if (ray_origin(u, k, px, py, pos) && ray_start(p, k, px, py, pos, s))
-        walk<FMT, false, CkptVisitor, 1, true>(p, k, s, vis,
-                                               PathSlots{&path_w[0][threadIdx.x], &path_p[0][threadIdx.x], 128, nullptr});
+    const bool alive = inside && ray_origin(u, k, px, py, pos) && ray_start(p, k, px, py, pos, s);
+    walk<FMT, false, CkptVisitor, UNIT, 1>(p, k, s, vis, path, alive);
+    if (!inside) return;
     if (p.color) p.color[pix] = s.dst;
     hdr[pix] = make_int2(vis.count, s.nsamples);
 }
+template <int FMT>
+__device__ __noinline__ void forward_pixel_box(const RaycastParams& p, int px, int py, int2* hdr, Ckpt* ckpt,
+                                               int per_ray) {
+    forward_pixel<FMT, false>(p, px, py, hdr, ckpt, per_ray, PathSlots{nullptr, 0, nullptr});
+}
 
-// 6 resident CTAs per SM (80 registers, fewer spills): on the paged 1080p
-// frames 5.73-5.78 ms against 5.83-6.02 at 7 CTAs and 6.18-6.21 at 8 (the
-// atomics' contention, not the walk's latency, bounds it).  F64: binary64
-// gradient rows; WSUM: the lanes of a cell summed before the atomics
-// (scatter_texels).
-template <int FMT, bool F64, bool WSUM>
-__global__ void __launch_bounds__(128, 6) backward_kernel(const __grid_constant__ RaycastParams p, const int2* hdr,
-                                                       const Ckpt* ckpt, int per_ray, const float4* dl_dcolor,
-                                                       const GradTarget gt) {
+// 7 resident CTAs (28 warps) per SM, at most 72 registers per thread: the
+// occupancy that measured fastest for the plain ray cast
+template <int FMT>
+__global__ void __launch_bounds__(128, 7) forward_ckpt_kernel(const __grid_constant__ RaycastParams p, int2* hdr,
+                                                           Ckpt* ckpt, int per_ray) {
     int px, py;
-    pixel_of_strided(px, py);
+    pixel_of(px, py);
+    __shared__ uint32_t path[kPathLevels][128];
+    if (unit_box(p.u))
+        forward_pixel<FMT, true>(p, px, py, hdr, ckpt, per_ray,
+                                 PathSlots{&path[0][threadIdx.x], 128, nullptr});
+    else
+        forward_pixel_box<FMT>(p, px, py, hdr, ckpt, per_ray);
+}
+
+// One pixel of the adjoint.  F64: binary64 gradient rows; WSUM: the lanes of a
+// cell summed before the atomics (scatter_texels).
+template <int FMT, bool F64, bool WSUM, bool UNIT>
+__device__ __forceinline__ void backward_pixel(const RaycastParams& p, int px, int py, const int2* hdr,
+                                               const Ckpt* ckpt, int per_ray, const float4* dl_dcolor,
+                                               const GradTarget& gt, const PathSlots& path) {
     const vv_uniforms& u = p.u;
-    if (px >= u.width || py >= u.height) return;
-    const size_t pix = (size_t)py * u.width + px;
-    const int2 h = hdr[pix];
+    const bool inside = px < u.width && py < u.height;
+    const size_t pix = inside ? (size_t)py * u.width + px : 0;
+    int2 h = make_int2(0, 0);
+    float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (inside) {
+        h = hdr[pix];
+        g = dl_dcolor[pix];
+    }
     const int C = h.x, total = h.y;
-    if (C == 0 || total == 0) return;
-    float4 g = dl_dcolor[pix];
-    if (g.x == 0.f && g.y == 0.f && g.z == 0.f && g.w == 0.f) return;
     bool ok = true;
-    const WalkConsts k = walk_consts(p, fetch_node<false>(p, 0, 0, 0, ok));
+    const WalkConsts k = walk_consts(p, UNIT ? __ldg(p.walk) : fetch_node<false>(p, 0, 0, 0, ok));
     RayState s0;
     F3 pos;
-    if (!ray_origin(u, k, px, py, pos)) return;
-    ray_start(p, k, px, py, pos, s0);  // direction and brick step of this ray
+    bool more = C != 0 && total != 0 && (g.x != 0.f || g.y != 0.f || g.z != 0.f || g.w != 0.f) &&
+                ray_origin(u, k, px, py, pos);
+    if (more) ray_start(p, k, px, py, pos, s0);  // direction of this ray
     const Ckpt* ck = ckpt + pix * (size_t)per_ray;
-    __shared__ uint2 path_w[kPathLevels][128];
-    __shared__ uint32_t path_p[kPathLevels][128];
     uint32_t c_slot = 0xFFFFFFFFu;  // the last slot scattered into and its gradient row
     int c_row = -1;
     ReplayVisitor rv;
     rv.gx = g.x;
     rv.gy = g.y;
     rv.gz = g.z;
-    for (int c = C - 1; c >= 0; --c) {
-        const Ckpt cc = ck[c];
-        const int a = (int)cc.c.x, b = c + 1 < C ? (int)ck[c + 1].c.x : total;
-        for (int m = (b - a - 1) / kPiece; m >= 0; --m) {
-            RayState s = s0;
+    // pieces of the ray's chunks, the last first.  The lanes of a warp take
+    // their pieces together: they meet before every replay and every scatter
+    // (left to itself each lane runs ahead on its own, at 8 threads a warp
+    // instruction instead of 15).
+    int c = C - 1, m = -1, a = 0, b = total;
+    while (__any_sync(0xFFFFFFFFu, more)) {
+        RayState s = s0;
+        if (more) {
+            const Ckpt cc = ck[c];
+            if (m < 0) {
+                a = (int)cc.c.x;
+                m = (b - a - 1) / kPiece;
+            }
             s.pos = f3(cc.a.x, cc.a.y, cc.a.z);
             s.dst = make_float4(cc.a.w, cc.b.x, cc.b.y, cc.b.z);
             s.iter = __float_as_int(cc.b.w);
             s.nsamples = a;
-            s.nptr_x = cc.c.y;
-            s.nptr_y = cc.c.z;
-            s.nptr_z = cc.c.w;
+            s.nptr = cc.c.y;
             rv.first = a + m * kPiece;
             rv.last = min(b, rv.first + kPiece);
             rv.n = 0;
-            walk<FMT, false, ReplayVisitor, 1, true>(
-                p, k, s, rv, PathSlots{&path_w[0][threadIdx.x], &path_p[0][threadIdx.x], 128, nullptr});
+        }
+        walk<FMT, false, ReplayVisitor, UNIT, 1>(p, k, s, rv, path, more);
+        __syncwarp();
+        if (more) {
             for (int j = rv.n - 1; j >= 0; --j) {
                 const float tj = rv.T[j];
                 const float t = fabsf(tj);
@@ -329,8 +354,36 @@ __global__ void __launch_bounds__(128, 6) backward_kernel(const __grid_constant_
                 // g.a -= dot(g, src), the products summed in the order x, y, z, w
                 g.w = g.w - (rv.r[j] + g.w * rv.a[j]);
             }
+            if (--m < 0) {
+                b = a;
+                more = --c >= 0;
+            }
         }
     }
+}
+template <int FMT, bool F64, bool WSUM>
+__device__ __noinline__ void backward_pixel_box(const RaycastParams& p, int px, int py, const int2* hdr,
+                                                const Ckpt* ckpt, int per_ray, const float4* dl_dcolor,
+                                                const GradTarget& gt) {
+    backward_pixel<FMT, F64, WSUM, false>(p, px, py, hdr, ckpt, per_ray, dl_dcolor, gt,
+                                          PathSlots{nullptr, 0, nullptr});
+}
+
+// 6 resident CTAs per SM (80 registers, fewer spills): on the paged 1080p
+// frames 5.73-5.78 ms against 5.83-6.02 at 7 CTAs and 6.18-6.21 at 8 (the
+// atomics' contention, not the walk's latency, bounds it).
+template <int FMT, bool F64, bool WSUM>
+__global__ void __launch_bounds__(128, 6) backward_kernel(const __grid_constant__ RaycastParams p, const int2* hdr,
+                                                       const Ckpt* ckpt, int per_ray, const float4* dl_dcolor,
+                                                       const __grid_constant__ GradTarget gt) {
+    int px, py;
+    pixel_of_strided(px, py);
+    __shared__ uint32_t path[kPathLevels][128];
+    if (unit_box(p.u))
+        backward_pixel<FMT, F64, WSUM, true>(p, px, py, hdr, ckpt, per_ray, dl_dcolor, gt,
+                                             PathSlots{&path[0][threadIdx.x], 128, nullptr});
+    else
+        backward_pixel_box<FMT, F64, WSUM>(p, px, py, hdr, ckpt, per_ray, dl_dcolor, gt);
 }
 
 // grad[e] += copy_k[e] for the extra copies k of the rows in use (all rows

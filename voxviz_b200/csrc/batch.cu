@@ -4,7 +4,7 @@
 // all views from a device work queue (one atomic counter; tiles numbered view
 // by view, row-major inside a view).  The views' RaycastParams (uniforms +
 // the pools of each view's octree) travel by value in the kernel's parameter
-// space, up to kMaxLaunchViews views per launch (88 with the 360-byte view
+// space, up to kMaxLaunchViews views per launch (60 with the 512-byte view
 // record; larger batches launch in chunks), so a
 // CTA reads its view's parameters from the constant bank as the single-view
 // ray cast does, and runs render_pixel, the vv_render ray cast, on every
@@ -33,7 +33,7 @@ struct BatchView {
 };
 
 // The views of one launch.  Kernel parameters may take 32,764 bytes.
-constexpr int kMaxLaunchViews = 88;  // 360 bytes each
+constexpr int kMaxLaunchViews = 60;  // 512 bytes each
 struct BatchParams {
     int n;            // views
     int total_tiles;  // tiles of all n views
@@ -53,8 +53,7 @@ __global__ void __launch_bounds__(TW * TH, 896 / (TW * TH))
     const BatchView* views = bp.v;
     const int nviews = bp.n, total_tiles = bp.total_tiles;
     __shared__ int s_tile, s_view, s_tx, s_ty;
-    __shared__ uint2 path_w[kPathLevels][TW * TH];
-    __shared__ uint32_t path_p[kPathLevels][TW * TH];
+    __shared__ uint32_t path[kPathLevels][TW * TH];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // each warp covers an 8x4 block of the tile (coherent descents)
     const int wx = (warp % (TW / 8)) * 8 + (lane & 7);
@@ -80,9 +79,7 @@ __global__ void __launch_bounds__(TW * TH, 896 / (TW * TH))
         if (s_tile >= total_tiles) return;
         const RaycastParams& sp = views[s_view].p;
         const int px = s_tx * TW + wx, py = s_ty * TH + wy;
-        if (px < sp.u.width && py < sp.u.height)
-            render_pixel<FMT, false, STEPS, true>(sp, px, py,
-                                                  PathSlots{&path_w[0][threadIdx.x], &path_p[0][threadIdx.x], TW * TH, nullptr});
+        render_pixel<FMT, false, STEPS>(sp, px, py, PathSlots{&path[0][threadIdx.x], TW * TH, nullptr});
         // every thread is done with s_* before thread 0 takes the next tile
         __syncthreads();
     }
@@ -188,11 +185,8 @@ static int batch_launch(vv_ctx* c, const vv_batch_view* views, int32_t n, const 
             std::memset(&v, 0, sizeof(v));
             v.p.u = *u;
             set_divisors(v.p);
-            v.p.nodes = t.nodes;
-            for (int a = 0; a < 3; ++a) {
-                v.p.node_dim[a] = t.dim[a];
-                v.p.slots[a] = bv.ctx->slots[a];
-            }
+            set_nodes(v.p, t.nodes, t.dim);
+            for (int a = 0; a < 3; ++a) v.p.slots[a] = bv.ctx->slots[a];
             v.p.bricks = bv.ctx->bricks;
             v.p.cell_mask = ctx_cell_mask(bv.ctx);
             v.p.jitter = bv.ctx->d_jitter;

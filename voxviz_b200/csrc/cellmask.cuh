@@ -7,7 +7,11 @@
 // channel's bit pattern zero.  Such a sample is exactly (0,0,0,0) whatever
 // its weights, and compositing it leaves the destination unchanged, so the
 // walk may take the zero without loading the texels.  729 cells in words
-// 0..22; words 23..31 are zero (128 bytes per slot, one L1 line).
+// 0..22 (128 bytes per slot, one L1 line).  Word 31 holds the cells that are
+// not all zero projected on each axis: bit x, bit 9 + y and bit 18 + z set for
+// such a cell (x, y, z), so a ray whose samples stay in slabs without any on
+// one axis passes the whole brick without a look at its cells.  The words
+// between are zero, and word 31 is zero in a download of the masks.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -20,6 +24,7 @@ namespace vv {
 
 constexpr int kCellMaskWords = 32;
 constexpr int kCellsPerAxis = 9;
+constexpr int kOccupancyWord = 31;
 
 // Whether texel i of the pool (format FMT, 1000 texels per slot) is zero in
 // every bit.
@@ -45,6 +50,10 @@ __device__ __forceinline__ bool texel_is_zero(const void* pool, size_t i) {
 // flags) holds texel q of the slot and the CTA has synchronised; writes the
 // slot's 32 mask words.
 __device__ __forceinline__ void write_cell_mask(const uint8_t* zero, uint32_t* __restrict__ out) {
+    __shared__ uint32_t occupied;
+    if (threadIdx.x == 0) occupied = 0u;
+    __syncthreads();
+    uint32_t occ = 0u;
     for (int base = 0; base < 32 * kCellMaskWords; base += blockDim.x) {
         const int c = base + (int)threadIdx.x;
         bool z = false;
@@ -53,11 +62,16 @@ __device__ __forceinline__ void write_cell_mask(const uint8_t* zero, uint32_t* _
             const int t = (zz * 10 + y) * 10 + x;
             z = (zero[t] & zero[t + 1] & zero[t + 10] & zero[t + 11] & zero[t + 100] & zero[t + 101] &
                  zero[t + 110] & zero[t + 111]) != 0;
+            if (!z) occ |= (1u << x) | (1u << (9 + y)) | (1u << (18 + zz));
         }
         const unsigned b = __ballot_sync(0xFFFFFFFFu, z);
         // each warp covers the 32 cells of one mask word
-        if ((threadIdx.x & 31u) == 0u && c < 32 * kCellMaskWords) out[c >> 5] = b;
+        if ((threadIdx.x & 31u) == 0u && c < 32 * kOccupancyWord) out[c >> 5] = b;
     }
+    occ = __reduce_or_sync(0xFFFFFFFFu, occ);
+    if ((threadIdx.x & 31u) == 0u && occ) atomicOr(&occupied, occ);
+    __syncthreads();
+    if (threadIdx.x == 0) out[kOccupancyWord] = occupied;
 }
 
 }  // namespace vv

@@ -238,7 +238,8 @@ int vv_nodepool_upload(vv_ctx* c, int32_t tree, const uint32_t* words, int32_t d
         t.nodes = nullptr;
     }
     if (!t.nodes) {
-        cudaError_t e = cudaMalloc(&t.nodes, cells * sizeof(uint2));
+        // the words and, behind them, the walk's records (walknode.h)
+        cudaError_t e = cudaMalloc(&t.nodes, 2 * cells * sizeof(uint2));
         if (e != cudaSuccess) {
             t.nodes = nullptr;
             return fail(c, VV_ERR_OOM, "cudaMalloc node pool");
@@ -337,6 +338,7 @@ int vv_brickpool_download_cell_masks(vv_ctx* c, uint32_t* words) {
     VV_CUDA(c, cudaMemcpyAsync(words, c->cell_mask, (size_t)c->total_slots * kCellMaskWords * sizeof(uint32_t),
                                cudaMemcpyDeviceToHost, c->stream));
     VV_CUDA(c, cudaStreamSynchronize(c->stream));
+    for (long long s = 0; s < c->total_slots; ++s) words[s * kCellMaskWords + kOccupancyWord] = 0u;
     return VV_OK;
 }
 
@@ -480,11 +482,8 @@ static int diff_params(vv_ctx* c, int32_t tree, const vv_uniforms* u, RaycastPar
     std::memset(&p, 0, sizeof(p));
     p.u = *u;
     set_divisors(p);
-    p.nodes = t.nodes;
-    for (int a = 0; a < 3; ++a) {
-        p.node_dim[a] = t.dim[a];
-        p.slots[a] = c->slots[a];
-    }
+    set_nodes(p, t.nodes, t.dim);
+    for (int a = 0; a < 3; ++a) p.slots[a] = c->slots[a];
     p.bricks = c->bricks;
     p.cell_mask = ctx_cell_mask(c);
     p.jitter = c->d_jitter;
@@ -637,10 +636,7 @@ int vv_render(vv_ctx* c, int32_t tree, const vv_uniforms* u, const vv_frame_out*
         std::memset(&p, 0, sizeof(p));
         p.u = *u;
         set_divisors(p);
-        p.nodes = t.nodes;
-        p.node_dim[0] = t.dim[0];
-        p.node_dim[1] = t.dim[1];
-        p.node_dim[2] = t.dim[2];
+        set_nodes(p, t.nodes, t.dim);
         p.bricks = c->bricks;
         p.cell_mask = ctx_cell_mask(c);
         p.slots[0] = c->slots[0];
@@ -657,7 +653,8 @@ int vv_render(vv_ctx* c, int32_t tree, const vv_uniforms* u, const vv_frame_out*
             p.grads = c->grads;
             p.grad_fmt = c->grad_fmt;
         }
-        if (c->raycast_mode == VV_RAYCAST_REFILL && !u->compute_lighting) {
+        // the refill form walks the unit box only
+        if (c->raycast_mode == VV_RAYCAST_REFILL && !u->compute_lighting && is_unit_box(*u)) {
             if (!c->d_refill_counter) VV_CUDA(c, cudaMalloc(&c->d_refill_counter, sizeof(unsigned int)));
             VV_CUDA(c, launch_raycast_refill(c->fmt, p, c->d_refill_counter, c->stream));
         } else if (c->raycast_mode == VV_RAYCAST_STAGED && !u->compute_lighting && c->fmt == VV_FMT_RGBA8) {
@@ -786,11 +783,8 @@ int vv_measure_footprint_views(vv_ctx* c, int32_t tree, const vv_uniforms* us, i
         std::memset(&p, 0, sizeof(p));
         p.u = us[i];
         set_divisors(p);
-        p.nodes = t.nodes;
-        for (int a = 0; a < 3; ++a) {
-            p.node_dim[a] = t.dim[a];
-            p.slots[a] = c->slots[a];
-        }
+        set_nodes(p, t.nodes, t.dim);
+        for (int a = 0; a < 3; ++a) p.slots[a] = c->slots[a];
         p.bricks = c->bricks;
         p.jitter = c->d_jitter;
         p.status = c->d_status;

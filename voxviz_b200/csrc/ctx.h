@@ -11,7 +11,7 @@
 namespace vv {
 
 struct DeviceTree {
-    uint2* nodes = nullptr;  // block-linear node pool
+    uint2* nodes = nullptr;  // block-linear node pool, then its walk records (walknode.h)
     int dim[3] = {0, 0, 0};
     size_t cells = 0;
 };

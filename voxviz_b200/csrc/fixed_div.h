@@ -39,4 +39,22 @@ VV_FIXED_DIV_HD float fixed_div(float a, float b, float y) {
 #endif
 }
 
+// a / b for any b > 0 from y = RN(1/b), by two of Markstein's corrections: q0
+// is within 1.5 ulp of the quotient (half an ulp from each of y and the
+// product, at most doubled, and half from rounding), the first correction
+// brings it within 1 ulp, and from a q within 1 ulp the theorem gives
+// RN(q + r*y) = RN(a/b) whatever b.  a and b normal, at least 2^-60, and the
+// quotient below 2^64, so that every step stays in the normal range.
+VV_FIXED_DIV_HD float markstein_div(float a, float b, float y) {
+#if defined(__CUDA_ARCH__)
+    const float q0 = __fmul_rn(a, y);
+    const float q1 = __fmaf_rn(__fmaf_rn(-b, q0, a), y, q0);
+    return __fmaf_rn(__fmaf_rn(-b, q1, a), y, q1);
+#else
+    const float q0 = a * y;
+    const float q1 = std::fma(std::fma(-b, q0, a), y, q0);
+    return std::fma(std::fma(-b, q1, a), y, q1);
+#endif
+}
+
 }  // namespace vv

@@ -35,11 +35,8 @@ __global__ void __launch_bounds__(128, 7) raycast_kernel(const __grid_constant__
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int px = blockIdx.x * 16 + (warp & 1) * 8 + (lane & 7);
     const int py = blockIdx.y * 8 + (warp >> 1) * 4 + (lane >> 3);
-    if (px >= p.u.width || py >= p.u.height) return;
-    __shared__ uint2 path_w[kPathLevels][128];
-    __shared__ uint32_t path_p[kPathLevels][128];
-    render_pixel<FMT, COUNT, 1, !COUNT, LIT>(p, px, py,
-                                             PathSlots{&path_w[0][threadIdx.x], &path_p[0][threadIdx.x], 128, nullptr});
+    __shared__ uint32_t path[kPathLevels][128];
+    render_pixel<FMT, COUNT, 1, LIT>(p, px, py, PathSlots{&path[0][threadIdx.x], 128, nullptr});
 }
 
 // The brick-staging form (RGBA8 pools): the pixels and walk of raycast_kernel,
@@ -52,11 +49,9 @@ __global__ void __launch_bounds__(128, 6) raycast_staged_kernel(const __grid_con
     __syncwarp();
     const int px = blockIdx.x * 16 + (warp & 1) * 8 + (lane & 7);
     const int py = blockIdx.y * 8 + (warp >> 1) * 4 + (lane >> 3);
-    if (px >= p.u.width || py >= p.u.height) return;
-    __shared__ uint2 path_w[kPathLevels][128];
-    __shared__ uint32_t path_p[kPathLevels][128];
-    render_pixel<VV_FMT_RGBA8, false, 1, true, false, true>(
-        p, px, py, PathSlots{&path_w[0][threadIdx.x], &path_p[0][threadIdx.x], 128, &stage[warp]});
+    __shared__ uint32_t path[kPathLevels][128];
+    render_pixel<VV_FMT_RGBA8, false, 1, false, true>(
+        p, px, py, PathSlots{&path[0][threadIdx.x], 128, &stage[warp]});
 }
 
 cudaError_t launch_raycast_staged(int fmt, const RaycastParams& p, cudaStream_t s) {
@@ -73,9 +68,8 @@ cudaError_t launch_raycast_staged(int fmt, const RaycastParams& p, cudaStream_t 
 template <int FMT>
 __global__ void __launch_bounds__(128, 7) raycast_refill_kernel(const __grid_constant__ RaycastParams p,
                                                                 unsigned int* counter) {
-    __shared__ uint2 path_w[kPathLevels][128];
-    __shared__ uint32_t path_p[kPathLevels][128];
-    render_refill<FMT>(p, counter, PathSlots{&path_w[0][threadIdx.x], &path_p[0][threadIdx.x], 128, nullptr});
+    __shared__ uint32_t path[kPathLevels][128];
+    render_refill<FMT>(p, counter, PathSlots{&path[0][threadIdx.x], 128, nullptr});
 }
 
 cudaError_t launch_raycast_refill(int fmt, const RaycastParams& p, unsigned int* counter, cudaStream_t s) {
@@ -304,12 +298,18 @@ __device__ __forceinline__ size_t block_linear(uint32_t x, uint32_t y, uint32_t 
     return blk * 8u + ((x & 1u) | ((y & 1u) << 1) | ((z & 1u) << 2));
 }
 
+// Node i's words and its walk record.
+__device__ __forceinline__ void write_node(uint2* __restrict__ nodes, size_t i, uint2 w, int dx, int dy, int dz) {
+    nodes[i] = w;
+    nodes[(size_t)dx * dy * dz + i] = make_uint2(walk_link(w.x, dx, dy, dz), w.y);
+}
+
 __global__ void node_upload_kernel(const uint2* __restrict__ grid, uint2* __restrict__ nodes, int dx, int dy,
                                    int dz) {
     const size_t total = (size_t)dx * dy * dz;
     for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < total; g += (size_t)gridDim.x * blockDim.x) {
         uint32_t x = (uint32_t)(g % dx), y = (uint32_t)((g / dx) % dy), z = (uint32_t)(g / ((size_t)dx * dy));
-        nodes[block_linear(x, y, z, dx, dy)] = grid[g];
+        write_node(nodes, block_linear(x, y, z, dx, dy), grid[g], dx, dy, dz);
     }
 }
 
@@ -333,7 +333,7 @@ __global__ void node_patch_kernel(const vv_node_patch* __restrict__ patches, int
         set_status(status, VV_ERR_BOUNDS);
         return;
     }
-    nodes[block_linear(q.x, q.y, q.z, dx, dy)] = make_uint2(q.word0, q.word1);
+    write_node(nodes, block_linear(q.x, q.y, q.z, dx, dy), make_uint2(q.word0, q.word1), dx, dy, dz);
 }
 
 __global__ void node_patch_staged_kernel(const vv_node_patch* patches, const volatile uint32_t* count,
@@ -349,7 +349,7 @@ __global__ void node_patch_staged_kernel(const vv_node_patch* patches, const vol
             set_status(status, VV_ERR_BOUNDS);
             continue;
         }
-        nodes[block_linear(q.x, q.y, q.z, dx, dy)] = make_uint2(q.word0, q.word1);
+        write_node(nodes, block_linear(q.x, q.y, q.z, dx, dy), make_uint2(q.word0, q.word1), dx, dy, dz);
     }
 }
 

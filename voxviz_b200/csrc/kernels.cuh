@@ -7,6 +7,8 @@
 #include <cmath>
 
 #include "../../include/voxviz_b200.h"
+#include "lod_bound.h"
+#include "walknode.h"
 
 namespace vv {
 
@@ -14,6 +16,8 @@ namespace vv {
 struct RaycastParams {
     vv_uniforms u;
     const uint2* nodes;      // node pool, block-linear: 8 nodes of a 2x2x2 cell contiguous
+    const uint2* walk;       // the same nodes as the walk reads them (walknode.h)
+    BlockDiv row, slice;     // node blocks per row and per slice of the grid
     int node_dim[3];         // node-pool grid dims (even)
     const void* bricks;      // brick pool, slot-major brick-linear texels
     int slots[3];            // slots per axis
@@ -31,15 +35,38 @@ struct RaycastParams {
     // 1 / ray_step_size when that is a power of two (else 0: divide)
     float rpdim[3];
     float rstep;
+    lodb::Consts lodk;       // set_divisors: constants of the LOD certificate (lod_bound.h)
+    float bstep_texel[3];    // set_divisors: texels a brick sample moves along a unit direction
     int color8;              // colour as RGBA8 unorm: color is read as uint32_t[H*W]
 };
 
-// The reciprocals of RaycastParams from its uniforms (host).
+// The node pool of a launch (host): its walk records follow its words.
+inline void set_nodes(RaycastParams& p, const uint2* nodes, const int dim[3]) {
+    p.nodes = nodes;
+    p.walk = nodes + (size_t)dim[0] * dim[1] * dim[2];
+    for (int a = 0; a < 3; ++a) p.node_dim[a] = dim[a];
+    p.row = make_block_div((uint32_t)dim[0] / 2u);
+    p.slice = make_block_div((uint32_t)dim[0] / 2u * ((uint32_t)dim[1] / 2u));
+}
+
+// Whether the volume box is [0,1]^3.
+inline bool is_unit_box(const vv_uniforms& u) {
+    for (int a = 0; a < 3; ++a)
+        if (u.vol_extent_min[a] != 0.0f || u.vol_extent_max[a] != 1.0f) return false;
+    return true;
+}
+
+// What RaycastParams holds derived from its uniforms (host).
 inline void set_divisors(RaycastParams& p) {
     for (int a = 0; a < 3; ++a) p.rpdim[a] = 1.0f / p.u.brick_pool_dimension[a];
     int e = 0;
     const float m = std::frexp(p.u.ray_step_size, &e);
     p.rstep = (m == 0.5f) ? 1.0f / p.u.ray_step_size : 0.0f;
+    const vv_uniforms& u = p.u;
+    const auto v3 = [](const float* f) { return lodb::V3{f[0], f[1], f[2]}; };
+    p.lodk = lodb::make_consts(v3(u.camera_position), v3(u.camera_up), v3(u.camera_left), u.root_voxel_half_size,
+                               u.lod_scalar, u.pixel_size, u.oct_tree_depth_minus_one, is_unit_box(u));
+    for (int a = 0; a < 3; ++a) p.bstep_texel[a] = u.brick_step_vector[a] * u.brick_pool_dimension[a];
 }
 
 // Pyramid/compaction launch state.

@@ -54,23 +54,11 @@ VV_HD V3 cross(V3 a, V3 b) { return V3{a.y * b.z - a.z * b.y, a.z * b.x - a.x * 
 
 VV_HD float fast_rsqrt(float x) {
 #ifdef __CUDA_ARCH__
-    return rsqrtf(x);
+    float r;  // x is a normal number wherever this is used
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
 #else
     return 1.0f / std::sqrt(x);
-#endif
-}
-VV_HD float fast_div(float a, float b) {
-#ifdef __CUDA_ARCH__
-    return __fdividef(a, b);
-#else
-    return a / b;
-#endif
-}
-VV_HD float fast_log2(float x) {
-#ifdef __CUDA_ARCH__
-    return __log2f(x);
-#else
-    return std::log2(x);
 #endif
 }
 VV_HD float vabs(float x) { return x < 0.0f ? -x : x; }
@@ -94,96 +82,133 @@ VV_HD float scale2(float x, int e) {
 #endif
 }
 
-// Per-ray constants.
+// Per-frame constants (made once on the host).
 struct Consts {
-    V3 C, w;       // camera position, w = up - left
-    float W, wn;   // |w|^2, |w| rounded up
-    float cmax;    // max |C| component
-    float rvh, lod, pixel_size;
+    V3 C, w;          // camera position, w = up - left
+    float W;          // |w|^2
+    float t0;         // 4 rvh |w| rounded up: t0 / |a| bounds 4 vh |w| / |a| at level 0
+    float ra_shallow; // 1/|a| up to which the levels above j0 are shown to continue (see clear_range)
+    float d0, d1;     // Dmax <= d0 / |a| + d1
+    float theta;      // theta <= theta * vh / |a|
+    float need;       // pixel_size / lod and the rounding terms: what R - theta Dmax has to reach
+    float guess;      // 0.97 rvh^2 / need
+    float rvh;
     int max_level;
     bool ok;
+    // deepest_clears: its level's half voxel size squared and times theta, the
+    // smallest |a|^2 it covers (0 / a huge one: none)
+    float quick_vh2, quick_theta, quick_min;
 };
 
+// Every rounding of a bound's own evaluation (a few ulp, approximate
+// reciprocal square roots included) is covered by the factors 1.001 on upper
+// and 1 - 3e-4 on lower bounds.
 VV_HD Consts make_consts(V3 C, V3 up, V3 left, float rvh, float lod, float pixel_size, int max_level, bool unit_box) {
+    const float u = 5.9604645e-8f;  // 2^-24
     Consts k;
     k.C = C;
     k.w = sub3(up, left);
     k.W = dot(k.w, k.w);
-    k.wn = (k.W > 0.0f ? 1.0f / fast_rsqrt(k.W) : 0.0f) * 1.0001f;
-    k.cmax = vmax(vabs(C.x), vmax(vabs(C.y), vabs(C.z)));
+    const float wn = (k.W > 0.0f ? 1.0f / fast_rsqrt(k.W) : 0.0f) * 1.001f;  // |w| rounded up
+    const float cmax = vmax(vabs(C.x), vmax(vabs(C.y), vabs(C.z)));
     k.rvh = rvh;
-    k.lod = lod;
-    k.pixel_size = pixel_size;
     k.max_level = max_level;
     k.ok = unit_box && lod > 0.0f && lod < 1e30f && pixel_size < 1e30f && rvh > 0.0f && k.W > 0.5f && k.W < 8.0f &&
-           k.cmax < 1e6f;
+           cmax < 1e6f;
+    k.t0 = 4.0f * rvh * wn * 1.001f;
+    // rounding of pos -+ uh +- lh - C per component with vh |w| <= |a|/4:
+    // u (2 max|pos| + max|a| + 5 vh + 2 cmax), max|a| <= |a|, 5 vh <= 1.25 |a| / |w|;
+    // e0 + e1 |a| bounds its norm
+    const float e0 = 1.7321f * u * (2.0f + 2.0f * cmax) * 1.02f;
+    const float e1 = 1.7321f * u * (1.0f + 1.25f * 1.003f / wn) * 1.02f;
+    k.d0 = 2.0f * 1.34f * e0 * 1.02f;
+    k.d1 = 2.0f * (1.34f * e1 + 1.8f * u) * 1.02f;
+    k.theta = 2.7f * wn * 1.001f;
+    const float px = pixel_size / lod;
+    k.need = px * (1.0f + 2e-4f) + 11.3f * u;
+    k.guess = k.need > 1e-30f ? 0.97f * rvh * rvh / k.need : 1e30f * rvh * rvh;
+    // levels above j0 (vh <= rvh there): a direction is off by at most
+    // 1.01 sqrt(3) eps / (0.316 |a|) + 1.8 u, eps = u (3 + 8 rvh + |a| + 2 cmax);
+    // both together move 1 - cos, which is over 0.0051, by s0 / |a| + s1
+    const float s0 = 2.0f * 1.01f * 1.7321f / 0.316f * u * (3.0f + 8.0f * rvh + 2.0f * cmax) * 1.02f;
+    const float s1 = 2.0f * (1.01f * 1.7321f / 0.316f * u + 1.8f * u) * 1.02f;
+    const float room = 0.0051f - s1 - 13.2f * u - px * (1.0f + 2e-4f);
+    k.ra_shallow = room > 0.0f ? room / s0 * (1.0f - 1e-3f) : 0.0f;
+    // the quick test of the deepest level: |a| at least 4 vh |w| there, and
+    // either no level above j0 or those shown; theta >= 5 Dmax from R >= need
+    const float vh = scale2(rvh, -max_level);
+    k.quick_vh2 = 2.0f * vh * vh * (1.0f - 6e-4f);
+    k.quick_theta = 1.001f * k.theta * vh;
+    float amin = 4.0f * vh * wn * 40.0f;  // (vh^2 W / A is then below 1/25600)
+    if (amin < k.t0) {
+        const float shallow = k.ra_shallow > 0.0f ? 1.001f / k.ra_shallow : 1e18f;
+        if (amin < shallow) amin = shallow < k.t0 ? shallow : k.t0;
+    }
+    const float dm = k.d0 / (amin > 1e-6f ? amin : 1e-6f) + k.d1;
+    k.quick_min = k.ok && max_level >= 0 && max_level < 60 && amin > 1e-6f && k.need >= 12.6f * dm * dm
+                      ? amin * amin * 1.001f : 3e38f;
     return k;
 }
 
+// Whether the LOD test surely continues at every level from 0 to max_level:
+// what clear_range shows for the deepest level, with |a| bounded by
+// (1 + |a|^2) / 2 in place of its square root.
+VV_HD bool deepest_clears(const Consts& k, V3 pos) {
+    const V3 a = sub3(pos, k.C);
+    const float A = dot(a, a);
+    const float aw = dot(a, k.w), AW = A * k.W;
+    const float S = AW - aw * aw;
+    return A >= k.quick_min && S >= 0.1002f * AW &&
+           k.quick_vh2 * S >= 1.0005f * A * (k.need * A + k.quick_theta * (k.d0 + k.d1 * (0.5f + 0.5f * A)));
+}
+
 // Levels [lo, hi] at which the LOD test surely continues for position pos
-// (inside the unit box); lo > hi when nothing is shown.  `guess` picks the
-// deepest level tried first (the level where Rlow is ~4x the threshold);
-// two levels are tried.
+// (inside the unit box); lo > hi when nothing is shown.  The deepest level is
+// picked from R ~ G vh^2 with 3 % to spare and, when its own bound falls
+// short (near the camera), the one above it.
 VV_HD void clear_range(const Consts& k, V3 pos, int& lo, int& hi) {
     lo = 1;
     hi = 0;
     if (!k.ok) return;
-    const float u = 5.9604645e-8f;  // 2^-24
     const V3 a = sub3(pos, k.C);
     const float A = dot(a, a);
-    if (!(A > 1e-12f)) return;
+    // |a x w|^2 = |a|^2 |w|^2 - (a.w)^2; with sin(angle(a, w)) >= 0.316 its
+    // cancellation leaves it within 1e-5
+    const float aw = dot(a, k.w), AW = A * k.W;
+    const float S = AW - aw * aw;
+    if (!(A > 1e-12f) || !(S >= 0.1002f * AW)) return;
     const float ra = fast_rsqrt(A);
-    // a lower bound on |a| (the 1e-4 covers the approximate reciprocal square
-    // root and division, <= 2 ulp each on the device)
-    const float alen_lo = fast_div(1.0f, ra * 1.0001f);
-    // j0: the smallest j with 2^j >= t = 4 rvh |w| / |a|
-    const float t = 4.0f * k.rvh * k.wn * ra * 1.001f;
+    const float invA = ra * ra;
+    // j0: the smallest j with 2^j >= t >= 4 rvh |w| / |a|
+    const float t = k.t0 * ra;
     int j0 = 0;
     if (t > 1.0f) {
         const uint32_t b = float_bits(t);
-        const int e = (int)((b >> 23) & 255u) - 127;  // t in [2^e, 2^(e+1))
-        j0 = (b & 0x7FFFFFu) ? e + 1 : e;
+        j0 = (int)((b >> 23) & 255u) - 126;  // t < 2^j0
     }
-    const V3 c = cross(a, k.w);
-    const float S = dot(c, c);
-    if (!(S >= 0.1001f * A * k.W)) return;  // sin(angle(a, w)) >= 0.316: a x w is well conditioned
-    const float amax = vmax(vabs(a.x), vmax(vabs(a.y), vabs(a.z)));
     // Levels below j0 (vh |w| > |a|/4): sin(theta) = 2|a||d| sin(phi) /
     // (|a - d||a + d|) >= 2 * 0.25 * 0.316 / 1.25^2 at vh |w| = |a|/4 and theta
-    // grows with vh, so R >= 1 - cos(0.101) > 0.0051.  |a -+ d| >= |a| sin(phi),
-    // so each direction of the binary32 sequence is off by at most
-    // 1.01 sqrt(3) eps_c / (0.316 |a|) + 1.8 u (eps_c: per-component rounding
-    // with vh <= rvh), which moves 1 - cos by at most that angle.
-    int lo_level = j0;
-    if (j0 > 0) {
-        const float eps_c = u * (3.0f + 8.0f * k.rvh + amax + 2.0f * k.cmax) * 1.01f;
-        // upper bounds below: approximate quotients are raised by 1e-6 (> 2 ulp)
-        const float dsh = 2.0f * (fast_div(1.01f * 1.7321f * eps_c, 0.316f * alen_lo) * 1.000001f + 1.8f * u);
-        if ((0.0051f - dsh - 13.2f * u) * k.lod * (1.0f - 2.0f * u) >= k.pixel_size * (1.0f + 1e-4f)) lo_level = 0;
-    }
-    const float eps = 1.7321f * u * (2.0f + amax + fast_div(1.25f * alen_lo, k.wn) * 1.000001f + 2.0f * k.cmax) * 1.01f;
-    const float dmax = 2.0f * (fast_div(1.34f * eps, alen_lo) * 1.000001f + 1.8f * u) * 1.01f;
-    if (lo_level == 0) {  // whatever the deeper levels give, [0, j0) is shown
+    // grows with vh, so R >= 1 - cos(0.101) > 0.0051, and |a -+ d| >= |a| sin(phi).
+    const bool shallow = j0 == 0 || ra <= k.ra_shallow;
+    if (shallow) {  // whatever the deeper levels give, [0, j0) is shown
         lo = 0;
         hi = j0 - 1;
     }
-    const float r0 = fast_div(2.0f * k.rvh * k.rvh * S, A * A);
-    const float q = fast_div(r0 * k.lod, 4.0f * vmax(k.pixel_size, 1e-30f));
-    if (!(q > 1.0f)) return;
-    int m = (int)(0.5f * fast_log2(q));
+    const float G = 2.0f * S * invA * invA;  // R ~ G vh^2
+    const float q = G * k.guess;
+    if (!(q >= 1.0f)) return;
+    int m = ((int)((float_bits(q) >> 23) & 255u) - 127) >> 1;  // floor(log2(q) / 2)
     m = m < k.max_level ? m : k.max_level;
+    const float dmax = k.d0 * ra + k.d1;
+    const float tm = k.theta * ra;
     for (int tries = 0; tries < 2 && m >= j0; ++tries, --m) {
         const float vh = scale2(k.rvh, -m);
         const float vh2 = vh * vh;
-        const float den = A + vh2 * k.W;
-        const float Rlow = fast_div(2.0f * vh2 * S, den * den) * (1.0f - 1e-4f);
-        const float theta_up = fast_div(2.7f * vh * k.wn, alen_lo) * 1.000001f;
-        const float x = 2.0f * Rlow;
-        const float theta_lo = x * fast_rsqrt(x) * (1.0f - 1e-4f);
-        if (!(theta_lo >= 5.0f * dmax)) continue;
-        const float margin = (Rlow - theta_up * dmax - 11.2f * u) * (1.0f - 1e-5f);
-        if (margin * k.lod * (1.0f - 4.0f * u) >= k.pixel_size * (1.0f + 1e-4f)) {
-            lo = lo_level;
+        // 2 vh^2 S / (A + vh^2 W)^2 >= G vh^2 (1 - 2 vh^2 W / A)
+        const float Rlow = G * vh2 * (1.0f - 2.0f * vh2 * k.W * invA) * (1.0f - 3e-4f);
+        // theta >= sqrt(2 R) >= 5 Dmax, and the bound itself
+        if (2.0f * Rlow >= 25.1f * dmax * dmax && Rlow - tm * vh * dmax * 1.001f >= k.need) {
+            lo = shallow ? 0 : j0;
             hi = m;
             return;
         }

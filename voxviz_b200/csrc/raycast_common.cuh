@@ -141,8 +141,95 @@ struct Texel<VV_FMT_DXT1> {
     }
 };
 
-__device__ __forceinline__ float4 lerp4(float4 a, float4 b, float t) {
-    return make_float4(lerpf(a.x, b.x, t), lerpf(a.y, b.y, t), lerpf(a.z, b.z, t), lerpf(a.w, b.w, t));
+// Two binary32 operations per instruction (sm_100a packed f32x2), each lane
+// rounded as the scalar operation rounds: the same values in half the issue
+// slots, which is what bounds the walk.
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// A texel as two channel pairs.
+struct Pair4 {
+    unsigned long long xy, zw;
+};
+__device__ __forceinline__ Pair4 pair4(float4 v) { return Pair4{pack2(v.x, v.y), pack2(v.z, v.w)}; }
+// lerpf of every channel, tt = (t, t)
+__device__ __forceinline__ Pair4 lerp4(Pair4 a, Pair4 b, unsigned long long tt) {
+    return Pair4{fma2(tt, sub2(b.xy, a.xy), a.xy), fma2(tt, sub2(b.zw, a.zw), a.zw)};
+}
+
+// The trilinear filter of eight texels (x fastest) with weights f, and the
+// format's scale.  RGBA8 texels come as 2^23 + byte: the x lerp's difference
+// of two of them is the bytes' difference exactly, so only its addend loses
+// the bias.
+template <int FMT>
+struct RawTexel {
+    using T = float4;
+    __device__ __forceinline__ static T load(const void* pool, uint32_t i) { return Texel<FMT>::load(pool, i); }
+    __device__ __forceinline__ static Pair4 lerp_x(T a, T b, unsigned long long tt) {
+        return lerp4(pair4(a), pair4(b), tt);
+    }
+};
+template <>
+struct RawTexel<VV_FMT_RGBA8> {
+    using T = uint32_t;
+    __device__ __forceinline__ static T load(const void* pool, uint32_t i) { return __ldg((const uint32_t*)pool + i); }
+    __device__ __forceinline__ static Pair4 biased(uint32_t v) {
+        return Pair4{pack2(__uint_as_float(__byte_perm(v, 0x4B000000u, 0x7440u)),
+                           __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7441u))),
+                     pack2(__uint_as_float(__byte_perm(v, 0x4B000000u, 0x7442u)),
+                           __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7443u)))};
+    }
+    __device__ __forceinline__ static Pair4 lerp_x(T a, T b, unsigned long long tt) {
+        const unsigned long long bias = pack2(-8388608.0f, -8388608.0f);
+        const Pair4 pa = biased(a), pb = biased(b);
+        return Pair4{fma2(tt, sub2(pb.xy, pa.xy), add2(pa.xy, bias)), fma2(tt, sub2(pb.zw, pa.zw), add2(pa.zw, bias))};
+    }
+};
+template <int FMT>
+__device__ __forceinline__ float4 filter8(const typename RawTexel<FMT>::T v[8], float fx, float fy, float fz) {
+    using R = RawTexel<FMT>;
+    const unsigned long long tx = pack2(fx, fx), ty = pack2(fy, fy), tz = pack2(fz, fz);
+    const Pair4 c0 = lerp4(R::lerp_x(v[0], v[1], tx), R::lerp_x(v[2], v[3], tx), ty);
+    const Pair4 c1 = lerp4(R::lerp_x(v[4], v[5], tx), R::lerp_x(v[6], v[7], tx), ty);
+    Pair4 c = lerp4(c0, c1, tz);
+    if (Texel<FMT>::kScale != 1.0f) {
+        const unsigned long long k = pack2(Texel<FMT>::kScale, Texel<FMT>::kScale);
+        c = Pair4{mul2(c.xy, k), mul2(c.zw, k)};
+    }
+    const float2 a = unpack2(c.xy), b = unpack2(c.zw);
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+// dst + T * src per channel (a product and a sum; the packed forms of the two
+// were seen to give the fused result, so they stay scalar)
+__device__ __forceinline__ float4 composite(float T, float4 src, float4 dst) {
+    return make_float4(T * src.x + dst.x, T * src.y + dst.y, T * src.z + dst.z, T * src.w + dst.w);
 }
 
 // One axis of GL_LINEAR + CLAMP_TO_EDGE (GL 3.3 spec 3.8.8): texel centres at
@@ -170,113 +257,99 @@ __device__ __forceinline__ Axis axis_taps(float u, float N, int n) {
 
 __device__ __forceinline__ void touch(uint32_t* bits, uint32_t i) { atomicOr(bits + (i >> 5), 1u << (i & 31u)); }
 
+// The trilinear fetch of the brick-pool texture at uvw, any taps.  Out of
+// line: the walk comes here only for samples whose taps leave their slot.
 template <int FMT, bool COUNT>
-__device__ __forceinline__ float4 sample_brick(const RaycastParams& p, F3 uvw) {
+__device__ __noinline__ float4 sample_brick(const RaycastParams& p, F3 uvw) {
     const float* N = p.u.brick_pool_dimension;
     const int nx = p.slots[0] * 10, ny = p.slots[1] * 10, nz = p.slots[2] * 10;
     Axis ax = axis_taps(uvw.x, N[0], nx);
     Axis ay = axis_taps(uvw.y, N[1], ny);
     Axis az = axis_taps(uvw.z, N[2], nz);
     const uint32_t SX = (uint32_t)p.slots[0], SY = (uint32_t)p.slots[1];
-    auto idx = [&](int sx, int lx, int sy, int ly, int sz, int lz) -> uint32_t {
-        uint32_t slot = ((uint32_t)sz * SY + (uint32_t)sy) * SX + (uint32_t)sx;
-        return slot * 1000u + (uint32_t)((lz * 10 + ly) * 10 + lx);
-    };
-    const void* pool = p.bricks;
-    float4 v000 = Texel<FMT>::load(pool, idx(ax.s0, ax.l0, ay.s0, ay.l0, az.s0, az.l0));
-    float4 v100 = Texel<FMT>::load(pool, idx(ax.s1, ax.l1, ay.s0, ay.l0, az.s0, az.l0));
-    float4 v010 = Texel<FMT>::load(pool, idx(ax.s0, ax.l0, ay.s1, ay.l1, az.s0, az.l0));
-    float4 v110 = Texel<FMT>::load(pool, idx(ax.s1, ax.l1, ay.s1, ay.l1, az.s0, az.l0));
-    float4 v001 = Texel<FMT>::load(pool, idx(ax.s0, ax.l0, ay.s0, ay.l0, az.s1, az.l1));
-    float4 v101 = Texel<FMT>::load(pool, idx(ax.s1, ax.l1, ay.s0, ay.l0, az.s1, az.l1));
-    float4 v011 = Texel<FMT>::load(pool, idx(ax.s0, ax.l0, ay.s1, ay.l1, az.s1, az.l1));
-    float4 v111 = Texel<FMT>::load(pool, idx(ax.s1, ax.l1, ay.s1, ay.l1, az.s1, az.l1));
-    if (COUNT) {
-        for (int k = 0; k < 8; ++k) {
-            const uint32_t sx = (uint32_t)((k & 1) ? ax.s1 : ax.s0), sy = (uint32_t)((k & 2) ? ay.s1 : ay.s0),
-                           sz = (uint32_t)((k & 4) ? az.s1 : az.s0);
-            touch(p.brick_touch, (sz * SY + sy) * SX + sx);
-        }
+    typename RawTexel<FMT>::T v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const uint32_t sx = (uint32_t)((k & 1) ? ax.s1 : ax.s0), sy = (uint32_t)((k & 2) ? ay.s1 : ay.s0),
+                       sz = (uint32_t)((k & 4) ? az.s1 : az.s0);
+        const int lx = (k & 1) ? ax.l1 : ax.l0, ly = (k & 2) ? ay.l1 : ay.l0, lz = (k & 4) ? az.l1 : az.l0;
+        const uint32_t slot = (sz * SY + sy) * SX + sx;
+        v[k] = RawTexel<FMT>::load(p.bricks, slot * 1000u + (uint32_t)((lz * 10 + ly) * 10 + lx));
+        if (COUNT) touch(p.brick_touch, slot);
     }
-    float4 c00 = lerp4(v000, v100, ax.f);
-    float4 c10 = lerp4(v010, v110, ax.f);
-    float4 c01 = lerp4(v001, v101, ax.f);
-    float4 c11 = lerp4(v011, v111, ax.f);
-    float4 c0 = lerp4(c00, c10, ay.f);
-    float4 c1 = lerp4(c01, c11, ay.f);
-    float4 c = lerp4(c0, c1, az.f);
-    if (Texel<FMT>::kScale != 1.0f) {
-        const float k = Texel<FMT>::kScale;
-        c = make_float4(c.x * k, c.y * k, c.z * k, c.w * k);
-    }
-    return c;
+    return filter8<FMT>(v, ax.f, ay.f, az.f);
 }
 
-// Trilinear sample when all 8 taps lie in the brick-pool slot whose first
-// texel per axis is base[]: kInSlot (out = the sample, same arithmetic as
-// sample_brick, only the texel addressing is shorter) or, when the slot's
-// cell mask `cmask` (or nullptr) marks the taps' cell all zero, kEmptyCell
-// (out = 0, exactly what the taps give); kOutside (and nothing) otherwise.
-// With STAGED and `stex` (the slot's RGBA8 texels in shared memory) the taps
-// are read from there.
-enum { kOutside = 0, kInSlot = 1, kEmptyCell = 2 };
-template <int FMT, bool STAGED = false>
-__device__ __forceinline__ int sample_in_slot(const RaycastParams& p, F3 uvw, const int base[3], uint32_t slot_texel0,
-                                              const uint32_t* cmask, float4& out, const uint32_t* stex = nullptr) {
-    const float* N = p.u.brick_pool_dimension;
-    const float ta[3] = {uvw.x * N[0] - 0.5f, uvw.y * N[1] - 0.5f, uvw.z * N[2] - 0.5f};
-    // the first tap per axis, floor(t) as an integer in one conversion (the
-    // weights below are only formed for a sample that is filtered)
+// The brick-pool slot a brick segment samples: its first texel per axis, its
+// first texel and its empty-cell mask (or nullptr).
+struct SlotView {
+    int bias[3];  // kFloorBits + first texel per axis
+    uint32_t texel0;
+    const uint32_t* cmask;
+};
+// floor(t) for |t| < 2^22 in one addition rounded down: the sum with 1.5 * 2^23
+// holds the integer in its low bits (a float-to-integer conversion runs at a
+// quarter of the rate).  Any other t gives an integer far outside a slot.
+constexpr float kFloorMagic = 12582912.0f;
+constexpr int kFloorBits = 0x4B400000;
+
+// Local index of the first tap of the sample at uvw per axis, in [0, 8] when
+// all eight taps lie in the slot; t (the texel coordinate) kept per axis.
+struct TapCell {
+    float t[3], fl[3];
     int l[3];
+    __device__ __forceinline__ TapCell(const RaycastParams& p, const SlotView& sv, F3 uvw) {
+        const float* N = p.u.brick_pool_dimension;
+        t[0] = uvw.x * N[0] - 0.5f;
+        t[1] = uvw.y * N[1] - 0.5f;
+        t[2] = uvw.z * N[2] - 0.5f;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) l[a] = __float2int_rd(ta[a]) - base[a];
-    if ((unsigned)l[0] > 8u || (unsigned)l[1] > 8u || (unsigned)l[2] > 8u) return kOutside;
-    if (cmask) {
-        const uint32_t c = (uint32_t)((l[2] * kCellsPerAxis + l[1]) * kCellsPerAxis + l[0]);
-        if ((__ldg(cmask + (c >> 5)) >> (c & 31u)) & 1u) {
-            out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            return kEmptyCell;
+        for (int a = 0; a < 3; ++a) {
+            fl[a] = __fadd_rd(t[a], kFloorMagic);
+            l[a] = __float_as_int(fl[a]) - sv.bias[a];
         }
     }
-    float f[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) f[a] = ta[a] - floorf(ta[a]);
-    const uint32_t l000 = (uint32_t)((l[2] * 10 + l[1]) * 10 + l[0]);
-    const uint32_t i000 = slot_texel0 + l000;
-    const void* pool = p.bricks;
-    float4 v000, v100, v010, v110, v001, v101, v011, v111;
+    __device__ __forceinline__ bool in_slot() const {
+        return max(max((unsigned)l[0], (unsigned)l[1]), (unsigned)l[2]) <= 8u;
+    }
+};
+
+// Whether the sample at uvw has to be fetched: false when its taps lie in the
+// slot and the slot's mask marks their cell all zero (the sample is then
+// exactly zero and compositing it changes nothing).
+__device__ __forceinline__ bool sample_needed(const RaycastParams& p, const SlotView& sv, F3 uvw) {
+    const TapCell c(p, sv, uvw);
+    const bool in = c.in_slot();
+    const uint32_t i = in ? (uint32_t)((c.l[2] * kCellsPerAxis + c.l[1]) * kCellsPerAxis + c.l[0]) : 0u;
+    const uint32_t w = __ldg(sv.cmask + (i >> 5));
+    return !(in && ((w >> (i & 31u)) & 1u));
+}
+
+// The sample at uvw: the in-slot filter (from stex, the slot's RGBA8 texels
+// in shared memory, when given), else the general one.
+template <int FMT, bool STAGED = false>
+__device__ __forceinline__ float4 fetch_sample(const RaycastParams& p, const SlotView& sv, F3 uvw,
+                                               const uint32_t* stex = nullptr) {
+    const TapCell c(p, sv, uvw);
+    if (!c.in_slot()) return sample_brick<FMT, false>(p, uvw);
+    const uint32_t l000 = (uint32_t)((c.l[2] * 10 + c.l[1]) * 10 + c.l[0]);
+    typename RawTexel<FMT>::T v[8];
     if (STAGED && stex) {
         static_assert(!STAGED || FMT == VV_FMT_RGBA8, "staging holds RGBA8 slots");
-        const uint32_t* t = stex + l000;
-        v000 = Texel<VV_FMT_RGBA8>::unpack(t[0]);
-        v100 = Texel<VV_FMT_RGBA8>::unpack(t[1]);
-        v010 = Texel<VV_FMT_RGBA8>::unpack(t[10]);
-        v110 = Texel<VV_FMT_RGBA8>::unpack(t[11]);
-        v001 = Texel<VV_FMT_RGBA8>::unpack(t[100]);
-        v101 = Texel<VV_FMT_RGBA8>::unpack(t[101]);
-        v011 = Texel<VV_FMT_RGBA8>::unpack(t[110]);
-        v111 = Texel<VV_FMT_RGBA8>::unpack(t[111]);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const uint32_t w = stex[l000 + (k & 1) + 10 * ((k >> 1) & 1) + 100 * (k >> 2)];
+            memcpy(&v[k], &w, sizeof(w));
+        }
     } else {
-        v000 = Texel<FMT>::load(pool, i000);
-        v100 = Texel<FMT>::load(pool, i000 + 1u);
-        v010 = Texel<FMT>::load(pool, i000 + 10u);
-        v110 = Texel<FMT>::load(pool, i000 + 11u);
-        v001 = Texel<FMT>::load(pool, i000 + 100u);
-        v101 = Texel<FMT>::load(pool, i000 + 101u);
-        v011 = Texel<FMT>::load(pool, i000 + 110u);
-        v111 = Texel<FMT>::load(pool, i000 + 111u);
+        const uint32_t i000 = sv.texel0 + l000;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            v[k] = RawTexel<FMT>::load(p.bricks, i000 + (k & 1) + 10 * ((k >> 1) & 1) + 100 * (k >> 2));
     }
-    const float4 c0 = lerp4(lerp4(v000, v100, f[0]), lerp4(v010, v110, f[0]), f[1]);
-    const float4 c1 = lerp4(lerp4(v001, v101, f[0]), lerp4(v011, v111, f[0]), f[1]);
-    float4 c = lerp4(c0, c1, f[2]);
-    if (Texel<FMT>::kScale != 1.0f) {
-        const float k = Texel<FMT>::kScale;
-        c = make_float4(c.x * k, c.y * k, c.z * k, c.w * k);
-    }
-    out = c;
-    return kInSlot;
+    return filter8<FMT>(v, c.t[0] - (c.fl[0] - kFloorMagic), c.t[1] - (c.fl[1] - kFloorMagic),
+                        c.t[2] - (c.fl[2] - kFloorMagic));
 }
-
 
 // A colour as RGBA8 unorm: round(clamp(c, 0, 1) * 255) per channel, to the
 // nearest (ties to even); NaN stores 0.
@@ -296,7 +369,7 @@ __device__ __forceinline__ float div_step(const RaycastParams& p, float t, float
 
 // ComputeMinRayBoxIntersection (GigaVoxelsNoLighting.frag:124-180): exit
 // time over the planes facing away from the ray, 4.0 if none, t == 0 ignored.
-__device__ __forceinline__ float min_exit(F3 p, F3 d, F3 mn, F3 mx) {
+static __device__ __noinline__ float min_exit(F3 p, F3 d, F3 mn, F3 mx) {
     float tmin = 4.0f;
     // planes 0..2: min faces with normals -x,-y,-z
     const float pa[3] = {p.x, p.y, p.z}, da[3] = {d.x, d.y, d.z};
@@ -320,6 +393,30 @@ __device__ __forceinline__ float min_exit(F3 p, F3 d, F3 mn, F3 mx) {
     return tmin;
 }
 
+// The exit time of one axis is num / |d|, num the distance to the plane ahead,
+// from y = exit_rcp(d) = RN(1 / |d|) (markstein_div, fixed_div.h: five
+// operations for the IEEE quotient).  exit_time takes the division for a num
+// below kExitSmall, and for |d| below 2^-60 any other num gives a quotient of
+// at least 4, which no exit time is: y = 0 then makes it 0, which exit_time
+// ignores the same way.
+constexpr float kExitSmall = 3.4694469519536142e-18f;  // 2^-58
+__device__ __forceinline__ float exit_rcp(float d) {
+    const float b = fabsf(d);
+    return b >= 8.6736173798840355e-19f ? 1.0f / b : 0.0f;  // 2^-60
+}
+// min_exit over the planes ahead of the ray (the only ones that face away
+// from it), `ahead` one plane per axis; three independent quotients.
+__device__ __forceinline__ float exit_time(F3 p, F3 d, F3 rinv, F3 lo, float size) {
+    const F3 num = f3(d.x < 0.0f ? p.x - lo.x : (lo.x + size) - p.x, d.y < 0.0f ? p.y - lo.y : (lo.y + size) - p.y,
+                      d.z < 0.0f ? p.z - lo.z : (lo.z + size) - p.z);
+    if (fminf(fminf(num.x, num.y), num.z) < kExitSmall)
+        return min_exit(p, d, lo, f3(lo.x + size, lo.y + size, lo.z + size));
+    const float tx = markstein_div(num.x, fabsf(d.x), rinv.x), ty = markstein_div(num.y, fabsf(d.y), rinv.y),
+                tz = markstein_div(num.z, fabsf(d.z), rinv.z);
+    // 0: an axis the ray does not move along
+    return fminf(fminf(tx != 0.0f ? tx : 4.0f, ty != 0.0f ? ty : 4.0f), fminf(tz != 0.0f ? tz : 4.0f, 4.0f));
+}
+
 __device__ __forceinline__ bool inside_box(F3 p, F3 mn, F3 mx) {
     return p.x > mn.x && p.y > mn.y && p.z > mn.z && mx.x > p.x && mx.y > p.y && mx.z > p.z;
 }
@@ -338,6 +435,30 @@ __device__ __forceinline__ uint2 fetch_node(const RaycastParams& p, uint32_t x, 
     return __ldg(p.nodes + idx);
 }
 
+// Grid position of node i of the pool.
+__device__ __forceinline__ void node_position(const RaycastParams& p, uint32_t i, uint32_t& x, uint32_t& y, uint32_t& z) {
+    const uint32_t blk = i >> 3, bz = block_div(blk, p.slice), r = blk - bz * p.slice.d, by = block_div(r, p.row);
+    x = 2u * (r - by * p.row.d) + (i & 1u);
+    y = 2u * by + ((i >> 1) & 1u);
+    z = 2u * bz + ((i >> 2) & 1u);
+}
+
+// The child of node `idx` at `depth` that holds pos, into idx, where the
+// walk's record does not give it (walknode.h: an odd or bad pointer) or the
+// position's fixed-point digits have run out; false out of the grid.
+static __device__ __noinline__ bool odd_child(const RaycastParams& p, F3 pos, int depth, uint32_t& idx) {
+    const float sc = pow2i(depth);
+    const F3 q = f3(pos.x * sc, pos.y * sc, pos.z * sc);
+    const uint32_t w = __ldg(&p.nodes[idx].x);
+    const uint32_t x = ((w >> 20) & 0x3FFu) + (q.x - floorf(q.x) >= 0.5f ? 1u : 0u),
+                   y = ((w >> 10) & 0x3FFu) + (q.y - floorf(q.y) >= 0.5f ? 1u : 0u),
+                   z = (w & 0x3FFu) + (q.z - floorf(q.z) >= 0.5f ? 1u : 0u);
+    if (x >= (uint32_t)p.node_dim[0] || y >= (uint32_t)p.node_dim[1] || z >= (uint32_t)p.node_dim[2]) return false;
+    const uint32_t bx = (uint32_t)p.node_dim[0] >> 1, by = (uint32_t)p.node_dim[1] >> 1;
+    idx = (((z >> 1) * by + (y >> 1)) * bx + (x >> 1)) * 8u + ((x & 1u) | ((y & 1u) << 1) | ((z & 1u) << 2));
+    return true;
+}
+
 // ---------------------------------------------------------------------------
 // The ray walk of GigaVoxelsNoLighting.frag main (:490-751) after the ray
 // set-up: leaf segments, each a descent from the root to the node that stops
@@ -349,29 +470,36 @@ __device__ __forceinline__ uint2 fetch_node(const RaycastParams& p, uint32_t x, 
 //   bool sample(int kind, float4 src, F3 bpos, float T, int index)
 //                                          before a sample is composited;
 //                                          false ends the walk after it
-//   void segment_end(const RayState&, bool is_const, bool loaded)
+//   void segment_end<UNIT>(const RaycastParams&, const RayState&)
 //   void fail(int code)
-// STEPS unrolls the two march loops (samples issued per loop trip); the
+// STEPS is the number of samples a march looks ahead (march_brick); the
 // results do not depend on it.
 
 struct WalkConsts {
     F3 C, vmin, vmax, up, left, bdim, pdim;
     float RS, astop, lod, pixel_size, rvh;
     int L, max_iter;
-    uint2 root;
-    lodb::Consts lodk;  // certificate constants of the LOD test (lod_bound.h)
-    bool unit_box;      // volume extent [0,1]^3 (as compute_uniforms derives it)
+    uint2 root;  // the root's walk record (unit box) or words
 };
 
 struct RayState {
-    F3 pos, dir, brick_step;
+    F3 pos, dir;
+    F3 rinv;        // exit_rcp of dir
     float4 dst;
     int iter;
-    int nsamples;                        // samples composited so far
-    uint32_t nptr_x, nptr_y, nptr_z;     // octTreeNodePtr (not reset between segments)
+    int nsamples;   // samples composited so far
+    // octTreeNodePtr (not reset between segments): in the unit box the index of
+    // the node, else x << 20 | y << 10 | z
+    uint32_t nptr;
 };
 
 enum { kSampleConst = 0, kSampleBrick = 1 };
+
+// Whether the volume box is [0,1]^3.
+__device__ __forceinline__ bool unit_box(const vv_uniforms& u) {
+    return u.vol_extent_min[0] == 0.0f && u.vol_extent_min[1] == 0.0f && u.vol_extent_min[2] == 0.0f &&
+           u.vol_extent_max[0] == 1.0f && u.vol_extent_max[1] == 1.0f && u.vol_extent_max[2] == 1.0f;
+}
 
 __device__ __forceinline__ WalkConsts walk_consts(const RaycastParams& p, uint2 root) {
     const vv_uniforms& u = p.u;
@@ -391,11 +519,6 @@ __device__ __forceinline__ WalkConsts walk_consts(const RaycastParams& p, uint2 
     k.L = u.oct_tree_depth_minus_one;
     k.max_iter = p.max_iter;
     k.root = root;
-    k.unit_box = k.vmin.x == 0.0f && k.vmin.y == 0.0f && k.vmin.z == 0.0f && k.vmax.x == 1.0f &&
-                 k.vmax.y == 1.0f && k.vmax.z == 1.0f;
-    k.lodk = lodb::make_consts(lodb::V3{k.C.x, k.C.y, k.C.z}, lodb::V3{k.up.x, k.up.y, k.up.z},
-                               lodb::V3{k.left.x, k.left.y, k.left.z}, k.rvh, k.lod, k.pixel_size, k.L,
-                               k.unit_box);
     return k;
 }
 
@@ -449,26 +572,25 @@ __device__ __forceinline__ bool ray_start(const RaycastParams& p, const WalkCons
     const int J = u.jitter_tex_size;
     const float jitter = (float)p.jitter[(py % J) * J + (px % J)] / 255.0f;
     s.pos = add(pos, muls(muls(s.dir, k.RS), jitter));
-    s.brick_step = mul(s.dir, ld3(u.brick_step_vector));
+    s.rinv = f3(exit_rcp(s.dir.x), exit_rcp(s.dir.y), exit_rcp(s.dir.z));
     s.dst = make_float4(0.f, 0.f, 0.f, 0.f);
     s.iter = 0;
     s.nsamples = 0;
-    s.nptr_x = s.nptr_y = s.nptr_z = 0u;
+    s.nptr = 0u;
     return inside_box(s.pos, k.vmin, k.vmax);
 }
 
-// The path of the ray's last descent, per thread in shared memory: node word
-// and packed grid position (x<<20 | y<<10 | z) of each level, `stride`
-// elements apart per level.  A later descent whose position lies in the same
-// level-r node, and whose LOD test lodb::clear_range shows to continue at
-// every level above r, starts at that node instead of the root: the levels
-// it skips would take exactly the recorded path (same nodes, same words,
-// every stop condition false), so the walk is unchanged.
+// The path of the ray's last descent, per thread in shared memory: the index
+// of the node of each level, `stride` elements apart per level.  A later
+// descent whose position lies in the same level-r node, and whose LOD test
+// lodb::clear_range shows to continue at every level above r, starts at that
+// node instead of the root: the levels it skips would take exactly the
+// recorded path (same nodes, every stop condition false), so the walk is
+// unchanged.
 constexpr int kPathLevels = 11;  // levels 0..10
 struct StageBuf;
 struct PathSlots {
-    uint2* w;
-    uint32_t* p;
+    uint32_t* node;
     int stride;
     StageBuf* stage;  // the warp's staged brick (VV_RAYCAST_STAGED), else nullptr
 };
@@ -595,26 +717,15 @@ __device__ __forceinline__ F3 sample_gradient(const RaycastParams& p, F3 uvw) {
     const Axis ay = axis_taps(uvw.y, N[1], p.slots[1] * 10);
     const Axis az = axis_taps(uvw.z, N[2], p.slots[2] * 10);
     const uint32_t SX = (uint32_t)p.slots[0], SY = (uint32_t)p.slots[1];
-    auto idx = [&](int sx, int lx, int sy, int ly, int sz, int lz) -> uint32_t {
-        const uint32_t slot = ((uint32_t)sz * SY + (uint32_t)sy) * SX + (uint32_t)sx;
-        return slot * 1000u + (uint32_t)((lz * 10 + ly) * 10 + lx);
-    };
-    const void* g = p.grads;
-    const float4 v000 = Texel<GFMT>::load(g, idx(ax.s0, ax.l0, ay.s0, ay.l0, az.s0, az.l0));
-    const float4 v100 = Texel<GFMT>::load(g, idx(ax.s1, ax.l1, ay.s0, ay.l0, az.s0, az.l0));
-    const float4 v010 = Texel<GFMT>::load(g, idx(ax.s0, ax.l0, ay.s1, ay.l1, az.s0, az.l0));
-    const float4 v110 = Texel<GFMT>::load(g, idx(ax.s1, ax.l1, ay.s1, ay.l1, az.s0, az.l0));
-    const float4 v001 = Texel<GFMT>::load(g, idx(ax.s0, ax.l0, ay.s0, ay.l0, az.s1, az.l1));
-    const float4 v101 = Texel<GFMT>::load(g, idx(ax.s1, ax.l1, ay.s0, ay.l0, az.s1, az.l1));
-    const float4 v011 = Texel<GFMT>::load(g, idx(ax.s0, ax.l0, ay.s1, ay.l1, az.s1, az.l1));
-    const float4 v111 = Texel<GFMT>::load(g, idx(ax.s1, ax.l1, ay.s1, ay.l1, az.s1, az.l1));
-    const float4 c0 = lerp4(lerp4(v000, v100, ax.f), lerp4(v010, v110, ax.f), ay.f);
-    const float4 c1 = lerp4(lerp4(v001, v101, ax.f), lerp4(v011, v111, ax.f), ay.f);
-    float4 c = lerp4(c0, c1, az.f);
-    if (Texel<GFMT>::kScale != 1.0f) {
-        const float kk = Texel<GFMT>::kScale;
-        c = make_float4(c.x * kk, c.y * kk, c.z * kk, c.w * kk);
+    typename RawTexel<GFMT>::T v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const uint32_t sx = (uint32_t)((k & 1) ? ax.s1 : ax.s0), sy = (uint32_t)((k & 2) ? ay.s1 : ay.s0),
+                       sz = (uint32_t)((k & 4) ? az.s1 : az.s0);
+        const int lx = (k & 1) ? ax.l1 : ax.l0, ly = (k & 2) ? ay.l1 : ay.l0, lz = (k & 4) ? az.l1 : az.l0;
+        v[k] = RawTexel<GFMT>::load(p.grads, ((sz * SY + sy) * SX + sx) * 1000u + (uint32_t)((lz * 10 + ly) * 10 + lx));
     }
+    const float4 c = filter8<GFMT>(v, ax.f, ay.f, az.f);
     return f3(c.x, c.y, c.z);
 }
 
@@ -649,244 +760,516 @@ __device__ __forceinline__ void light_sample(const RaycastParams& p, F3 bpos, F3
     src.z = src.z + sh.z;
 }
 
-// Where a ray's last descent stopped (RESUME): its depth and its node's
-// cell there, packed 10:10:10.
+// The lower corner of the depth-d node of the unit box that holds pos, whose
+// fixed-point form (1 + pos rounded to zero, see walk_round_unit) is ix, iy, iz.
+__device__ __forceinline__ F3 unit_corner(F3 pos, uint32_t ix, uint32_t iy, uint32_t iz, int d) {
+    if (d <= 23) {
+        const uint32_t m = 0xFFFFFFFFu << (23 - d);
+        return f3(__uint_as_float(ix & m) - 1.0f, __uint_as_float(iy & m) - 1.0f, __uint_as_float(iz & m) - 1.0f);
+    }
+    const float sc = pow2i(d), rs = pow2i(-d);
+    return f3(floorf(pos.x * sc) * rs, floorf(pos.y * sc) * rs, floorf(pos.z * sc) * rs);
+}
+
+// The slot whose texels a brick pointer covers with a border of one (slot
+// origin + 1 per axis), or kNoSlot for another pointer.
+__device__ __forceinline__ uint32_t slot_of(const RaycastParams& p, uint32_t bw) {
+    const uint32_t x = (bw >> 20) & 0x3FFu, y = (bw >> 10) & 0x3FFu, z = bw & 0x3FFu;
+    const uint32_t sx = (x - 1u) / 10u, sy = (y - 1u) / 10u, sz = (z - 1u) / 10u;  // (a pointer of 0 wraps)
+    if (sx * 10u + 1u != x || sy * 10u + 1u != y || sz * 10u + 1u != z || sx >= (uint32_t)p.slots[0] ||
+        sy >= (uint32_t)p.slots[1] || sz >= (uint32_t)p.slots[2])
+        return kNoSlot;
+    return (sz * (uint32_t)p.slots[1] + sy) * (uint32_t)p.slots[0] + sx;
+}
+
+// Whether n samples of a brick segment that enters its node at the relative
+// position brp all fall in empty cells of slot `slot`, by the projections of
+// the occupied cells (cellmask.cuh).  The texel coordinates of the first and
+// the last sample bound those between, per axis; they are off from the
+// shader's sums by less than 0.01 texel for up to 128 samples (a sum of
+// coordinates below 1 in pools of at most 1020 texels rounds by 6e-5 texel).
+__device__ __forceinline__ bool brick_empty(const RaycastParams& p, const WalkConsts& k, F3 brp, F3 dir, int n,
+                                            uint32_t slot) {
+    const uint32_t occ = __ldg(p.cell_mask + (size_t)slot * kCellMaskWords + kOccupancyWord);
+    const float m = (float)(n - 1);
+    const F3 u0 = f3(fmaf(brp.x, k.bdim.x, 0.5f), fmaf(brp.y, k.bdim.y, 0.5f), fmaf(brp.z, k.bdim.z, 0.5f));
+    const F3 u1 = f3(fmaf(m * dir.x, p.bstep_texel[0], u0.x), fmaf(m * dir.y, p.bstep_texel[1], u0.y),
+                     fmaf(m * dir.z, p.bstep_texel[2], u0.z));
+    bool in = n <= 128, empty = false;
+    const float a0[3] = {u0.x, u0.y, u0.z}, a1[3] = {u1.x, u1.y, u1.z};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float lo = fminf(a0[a], a1[a]) - 0.02f, hi = fmaxf(a0[a], a1[a]) + 0.02f;
+        in = in && lo >= 0.0f && hi < 9.0f;
+        // bits of the slabs [floor(lo), floor(hi)], by the floor of TapCell
+        const int l = __float_as_int(__fadd_rd(lo, kFloorMagic)) & 15, h = __float_as_int(__fadd_rd(hi, kFloorMagic)) & 15;
+        empty = empty || (((2u << h) - (1u << l)) & (occ >> (9 * a)) & 0x1FFu) == 0u;
+    }
+    return in && empty;
+}
+
+// A brick segment about to be marched (TraverseBrick, :311-359): the first
+// sample's brick-pool position, the steps and the slot.
+struct BrickMarch {
+    F3 bpos, bstep, wstep;
+    float step;
+    int n;  // samples to the exit
+    uint32_t slot_id;
+    SlotView sv;
+    // bw: the brick's pool pointer; brp: the relative position in its node
+    template <bool COUNT>
+    __device__ __forceinline__ void set(const RaycastParams& p, const WalkConsts& k, const RayState& s, uint32_t bw, F3 brp,
+                                        int brick_depth, float t) {
+        // the six quotients by the pool dimensions from their reciprocals (fixed_div.h)
+        const uint32_t ptr[3] = {(bw >> 20) & 0x3FFu, (bw >> 10) & 0x3FFu, bw & 0x3FFu};
+        const F3 bptr = f3(fixed_div((float)ptr[0], k.pdim.x, p.rpdim[0]), fixed_div((float)ptr[1], k.pdim.y, p.rpdim[1]),
+                           fixed_div((float)ptr[2], k.pdim.z, p.rpdim[2]));
+        const F3 brb = mul(brp, k.bdim);
+        bpos = add(bptr, f3(fixed_div(brb.x, k.pdim.x, p.rpdim[0]), fixed_div(brb.y, k.pdim.y, p.rpdim[1]),
+                            fixed_div(brb.z, k.pdim.z, p.rpdim[2])));
+        const float ratio = pow2i(k.L - brick_depth);
+        wstep = muls(muls(s.dir, k.RS), ratio);
+        bstep = mul(s.dir, ld3(p.u.brick_step_vector));
+        step = k.RS * ratio;
+        n = (int)div_step(p, t, step, k.L - brick_depth) + 1;
+        // taps inside this brick's slot skip the general texel addressing
+        sv.texel0 = 0u;
+        sv.cmask = nullptr;  // (not in footprint counts)
+        sv.bias[0] = sv.bias[1] = sv.bias[2] = 0;  // no texel coordinate is in this slot
+        slot_id = slot_of(p, bw);
+        if (slot_id != kNoSlot) {
+            sv.texel0 = slot_id * 1000u;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) sv.bias[a] = kFloorBits - 1 + (int)ptr[a];
+            if (!COUNT && p.cell_mask) sv.cmask = p.cell_mask + (size_t)slot_id * kCellMaskWords;
+        }
+    }
+};
+// A brick segment whose samples are all in empty cells is stepped over: the
+// position takes the shader's sums, nothing is composited.  False, and nothing
+// done, when that is not shown.
+__device__ __forceinline__ bool step_over_brick(const RaycastParams& p, const WalkConsts& k, RayState& s, F3 corner,
+                                                uint32_t bw, int brick_depth, float t) {
+    const uint32_t slot = slot_of(p, bw);
+    if (slot == kNoSlot) return false;
+    const float ratio = pow2i(k.L - brick_depth);
+    const int n = (int)div_step(p, t, k.RS * ratio, k.L - brick_depth) + 1;
+    if (!brick_empty(p, k, muls(sub(s.pos, corner), pow2i(brick_depth)), s.dir, n, slot)) return false;
+    const F3 wstep = muls(muls(s.dir, k.RS), ratio);
+    for (int i = 0; i < n; ++i) s.pos = add(s.pos, wstep);
+    s.nsamples += n;
+    return true;
+}
+
+// lightDir = normalize(LightPosition - rayWorldPosition) at entry (:337)
+template <bool LIT>
+__device__ __forceinline__ F3 entry_light(const RaycastParams& p, const RayState& s) {
+    return LIT ? normalize3(sub(ld3(p.u.light_position), s.pos)) : f3(0.0f, 0.0f, 0.0f);
+}
+// One sample composited; false when the visitor ends the walk after it.
+template <bool LIT, class V>
+__device__ __forceinline__ bool take_sample(const RaycastParams& p, RayState& s, V& vis, float4 src, F3 bpos, F3 light_dir) {
+    src.w = 1.0f - (1.0f - src.w);
+    if (LIT) light_sample(p, bpos, s.dir, light_dir, src);
+    const float T = 1.0f - s.dst.w;
+    const bool go = vis.sample(kSampleBrick, src, bpos, T, s.nsamples);
+    s.dst = composite(T, src, s.dst);
+    ++s.nsamples;
+    return go;
+}
+
+// The march, a lane on its own; false when the visitor ends the walk.
+template <int FMT, bool COUNT, class V, bool LIT>
+__device__ __forceinline__ bool march_brick(const RaycastParams& p, const WalkConsts& k, RayState& s, V& vis, BrickMarch& b) {
+    const F3 light_dir = entry_light<LIT>(p, s);
+    bool go = true;
+    for (int i = 0; i < b.n && go; ++i) {
+        s.pos = add(s.pos, b.wstep);
+        if (s.dst.w > k.astop) {
+            s.pos = add(s.pos, muls(s.dir, (float)(b.n - (i + 1)) * b.step));
+            break;
+        }
+        const float4 src = COUNT ? sample_brick<FMT, COUNT>(p, b.bpos) : fetch_sample<FMT>(p, b.sv, b.bpos);
+        go = take_sample<LIT>(p, s, vis, src, b.bpos, light_dir);
+        b.bpos = add(b.bpos, b.bstep);
+    }
+    return go;
+}
+
+// The march of the lanes `lanes` of a warp together.  Most samples fall in
+// empty cells: each lane steps over them by the position sums alone (the
+// shader's, one per step and in its order) to its next sample that has to be
+// fetched, where the lanes meet.  The warp then filters once for all of them:
+// as often as its busiest lane needs it, not at every step at which any lane
+// does.  AHEAD cells are tested at a time, their mask loads in flight together.
+template <int FMT, class V, int AHEAD, bool LIT, bool STAGED>
+__device__ __forceinline__ bool march_brick_warp(const RaycastParams& p, const WalkConsts& k, RayState& s, V& vis,
+                                                 BrickMarch& b, unsigned lanes, StageBuf* stage) {
+    const F3 light_dir = entry_light<LIT>(p, s);
+    const bool staged = STAGED && stage_acquire(stage, p.bricks, b.slot_id, p.status);
+    const uint32_t* stex = staged ? stage->texels : nullptr;
+    bool go = true;
+    int left = b.n;  // samples not yet taken
+    if (left > 0 && s.dst.w > k.astop) {  // opaque before the first one: the ray moves to the exit
+        s.pos = add(add(s.pos, b.wstep), muls(s.dir, (float)(left - 1) * b.step));
+        left = 0;
+    }
+    int ahead = 0;        // of those left, tested
+    uint32_t needed = 0;  // bit j: the j-th of the tested has to be fetched
+    while (__any_sync(lanes, left > 0)) {
+        bool need = left > 0;
+        if (!V::kEverySample && need && b.sv.cmask) {
+            if (AHEAD == 1) {
+                while (left > 0 && !sample_needed(p, b.sv, b.bpos)) {
+                    s.pos = add(s.pos, b.wstep);
+                    b.bpos = add(b.bpos, b.bstep);
+                    ++s.nsamples;
+                    --left;
+                }
+                need = left > 0;
+            } else {
+                for (;;) {
+                    if (ahead == 0) {
+                        F3 q = b.bpos;
+                        needed = 0u;
+#pragma unroll
+                        for (int j = 0; j < AHEAD; ++j) {
+                            if (sample_needed(p, b.sv, q)) needed |= 1u << j;
+                            q = add(q, b.bstep);
+                        }
+                        ahead = min(AHEAD, left);
+                        needed &= (1u << ahead) - 1u;
+                    }
+                    const int skip = needed ? __ffs(needed) - 1 : ahead;
+                    for (int j = 0; j < skip; ++j) {
+                        s.pos = add(s.pos, b.wstep);
+                        b.bpos = add(b.bpos, b.bstep);
+                    }
+                    s.nsamples += skip;
+                    left -= skip;
+                    ahead -= skip;
+                    needed >>= skip;
+                    if (needed || left == 0) break;
+                }
+                need = left > 0;
+                --ahead;
+                needed >>= 1;
+            }
+        }
+        __syncwarp(lanes);
+        if (need) {
+            s.pos = add(s.pos, b.wstep);
+            float4 src = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (!V::kEverySample || !b.sv.cmask || sample_needed(p, b.sv, b.bpos))
+                src = fetch_sample<FMT, STAGED>(p, b.sv, b.bpos, stex);
+            go = take_sample<LIT>(p, s, vis, src, b.bpos, light_dir);
+            b.bpos = add(b.bpos, b.bstep);
+            --left;
+            if (left > 0 && s.dst.w > k.astop) {  // the step at which the stop is seen, then the rest at once
+                s.pos = add(add(s.pos, b.wstep), muls(s.dir, (float)(left - 1) * b.step));
+                left = 0;
+            }
+            if (!go) left = 0;
+        }
+    }
+    if (staged) stage_release(stage);
+    return go;
+}
+
+// TraverseConstant (:230-282) of a node at `depth`, to the exit time t.  An
+// empty node (alpha / 255 < 0.005) is stepped over; the samples of another are
+// composited: false when the visitor ends the walk.
+__device__ __forceinline__ bool constant_empty(uint32_t w1) { return (w1 >> 24) < 2u; }
+__device__ __forceinline__ void step_over_constant(const RaycastParams& p, const WalkConsts& k, RayState& s, int depth,
+                                                   float t) {
+    const float step = k.RS * pow2i(k.L - depth);
+    const int n = (int)div_step(p, t, step, k.L - depth) + 1;
+    s.pos = add(s.pos, muls(s.dir, (float)n * step));
+}
+template <class V>
+__device__ __forceinline__ bool march_constant(const RaycastParams& p, const WalkConsts& k, RayState& s, V& vis,
+                                               uint32_t w1, int depth, float t) {
+    const float ratio = pow2i(k.L - depth);
+    const float step = k.RS * ratio;
+    const int n = (int)div_step(p, t, step, k.L - depth) + 1;
+    bool go = true;
+    const float aw = (float)(w1 >> 24) / 255.0f;
+    const F3 wstep = muls(s.dir, step);
+    const float sa = 1.0f - pow_pow2(1.0f - aw, k.L - depth);
+    const float4 src = make_float4((float)(w1 & 255u) / 255.0f * ratio, (float)((w1 >> 8) & 255u) / 255.0f * ratio,
+                                   (float)((w1 >> 16) & 255u) / 255.0f * ratio, sa);
+    for (int i = 0; i < n && go; ++i) {
+        s.pos = add(s.pos, wstep);
+        if (s.dst.w > k.astop) {
+            const int rem = n - (i + 1);
+            s.pos = add(s.pos, muls(s.dir, (float)rem * step));
+            break;
+        }
+        const float T = 1.0f - s.dst.w;
+        go = vis.sample(kSampleConst, src, s.pos, T, s.nsamples);
+        s.dst = composite(T, src, s.dst);
+        ++s.nsamples;
+    }
+    return go;
+}
+
+// ComputeVoxelSize (:429-441) * LodScalar against PixelSize, in the shader's
+// order: whether the descent stops at a node of half voxel size vhalf.
+__device__ __forceinline__ bool lod_stops(const WalkConsts& k, F3 pos, float vhalf) {
+    const F3 uh = muls(k.up, vhalf), lh = muls(k.left, vhalf);
+    const F3 ll = normalize3(sub(add(sub(pos, uh), lh), k.C));
+    const F3 ur = normalize3(sub(sub(add(pos, uh), lh), k.C));
+    const float proj = (1.0f - dot3(ll, ur)) * k.lod;
+    return k.pixel_size > proj;
+}
+
+// One leaf segment in a volume box other than [0,1]^3, or with footprint
+// counts: the descent from the root with the node's extent and the relative
+// position tracked in binary32 as the shader does.
+template <int FMT, bool COUNT, class V, bool LIT>
+__device__ __forceinline__ bool walk_segment_box(const RaycastParams& p, const WalkConsts& k, RayState& s, V& vis) {
+    if (!vis.segment_begin(s)) return false;
+    bool ok = true;
+    uint2 node = k.root;
+    F3 ext_min = k.vmin, ext_max = k.vmax;
+    float node_size = 1.0f, vhalf = k.rvh;
+    F3 rbp = s.pos, cur_brp = s.pos;
+    uint32_t cur_bw = k.root.y;
+    int depth = 0, brick_depth = 0;
+    bool is_const, loaded;
+    for (;;) {
+        if (++s.iter > k.max_iter) {
+            vis.fail(VV_ERR_TIMEOUT);
+            return false;
+        }
+        is_const = (node.x & kConstant) != 0u;
+        loaded = (node.x & kResident) != 0u;
+        if (loaded) {
+            cur_bw = node.y;
+            cur_brp = rbp;
+            brick_depth = depth;
+        }
+        const uint32_t cx = (node.x >> 20) & 0x3FFu, cy = (node.x >> 10) & 0x3FFu, cz = node.x & 0x3FFu;
+        if ((!is_const && !loaded) || (cx == 0u && cy == 0u && cz == 0u)) break;
+        if (lod_stops(k, s.pos, vhalf)) break;
+        const F3 boff = muls(rbp, 2.0f);
+        const uint32_t ox = boff.x >= 1.0f ? 1u : 0u;
+        const uint32_t oy = boff.y >= 1.0f ? 1u : 0u;
+        const uint32_t oz = boff.z >= 1.0f ? 1u : 0u;
+        rbp = sub(boff, f3((float)ox, (float)oy, (float)oz));
+        const uint32_t x = cx + ox, y = cy + oy, z = cz + oz;
+        ++depth;
+        node_size = node_size * 0.5f;
+        ext_min = add(ext_min, muls(f3((float)ox, (float)oy, (float)oz), node_size));
+        ext_max = sub(ext_max, muls(f3(1.0f - (float)ox, 1.0f - (float)oy, 1.0f - (float)oz), node_size));
+        vhalf = vhalf * 0.5f;
+        node = fetch_node<COUNT>(p, x, y, z, ok);
+        if (!ok) {
+            vis.fail(VV_ERR_BOUNDS);
+            return false;
+        }
+        s.nptr = (x << 20) | (y << 10) | z;
+    }
+    const float t = min_exit(s.pos, s.dir, ext_min, ext_max);
+    if (is_const) {
+        if (constant_empty(node.y)) step_over_constant(p, k, s, depth, t);
+        else if (!march_constant(p, k, s, vis, node.y, depth, t)) return false;
+    } else {
+        BrickMarch b;
+        b.set<COUNT>(p, k, s, cur_bw, cur_brp, brick_depth, t);
+        if (!march_brick<FMT, COUNT, V, LIT>(p, k, s, vis, b)) return false;
+    }
+    vis.template segment_end<false>(p, s);
+    if (s.dst.w > k.astop && (is_const || loaded)) return false;
+    // restart from the root (:688-720); the node pointer keeps its value
+    return inside_box(s.pos, k.vmin, k.vmax);
+}
+// Where a ray's last descent stopped: its depth (0: no path kept), the fixed-point
+// position it was made for and the levels of its path that hold a brick.
 struct WalkResume {
-    int prev_depth = -1;
-    uint32_t prev_cell = 0u;
+    int prev_depth = 0;
+    uint32_t ix = 0u, iy = 0u, iz = 0u, res = 0u;
 };
 
-// One leaf segment of the walk (a descent and its march); false when the
-// walk has ended.  walk() runs it until then.
-template <int FMT, bool COUNT, class V, int STEPS = 1, bool RESUME = false, bool LIT = false, bool STAGED = false>
-__device__ __forceinline__ bool walk_segment(const RaycastParams& p, const WalkConsts& k, RayState& s, V& vis,
-                                             PathSlots path, WalkResume& wr) {
-    bool ok = true;
-    int& prev_depth = wr.prev_depth;
-    uint32_t& prev_cell = wr.prev_cell;
-    {
-        if (!vis.segment_begin(s)) return false;
-        int skip_lo, skip_hi;
-        lodb::clear_range(k.lodk, lodb::V3{s.pos.x, s.pos.y, s.pos.z}, skip_lo, skip_hi);
-        uint2 node = k.root;
-        F3 ext_min = k.vmin, ext_max = k.vmax;
-        float node_size = 1.0f, vhalf = k.rvh;
-        // In the unit box the node's extent is its integer cell times 2^-depth
-        // exactly (the sums below add distinct powers of two), so the cell is
-        // tracked instead and the extent formed once after the descent.
-        uint32_t ccx = 0u, ccy = 0u, ccz = 0u;
-        F3 rbp = s.pos, cur_brp = s.pos;
-        uint32_t cur_bw = k.root.y;
-        int depth = 0, brick_depth = 0;
-        bool is_const, loaded;
-        if (RESUME && !COUNT && k.unit_box && prev_depth > 0 && prev_depth < kPathLevels && skip_lo == 0) {
-            // the deepest level whose node holds both this and the last position
-            const float sc = pow2i(prev_depth);
-            const uint32_t nx = (uint32_t)(s.pos.x * sc), ny = (uint32_t)(s.pos.y * sc),
-                           nz = (uint32_t)(s.pos.z * sc);
-            const uint32_t diff = (nx ^ (prev_cell >> 20)) | (ny ^ ((prev_cell >> 10) & 0x3FFu)) |
-                                  (nz ^ (prev_cell & 0x3FFu));
-            int r = prev_depth - (diff ? 32 - __clz(diff) : 0);
-            r = min(r, skip_hi + 1);
-            if (r >= 1 && s.iter + r <= k.max_iter) {
-                node = path.w[r * path.stride];
-                const uint32_t pp = path.p[r * path.stride];
-                s.nptr_x = pp >> 20;
-                s.nptr_y = (pp >> 10) & 0x3FFu;
-                s.nptr_z = pp & 0x3FFu;
-                depth = r;
-                vhalf = k.rvh * pow2i(-r);
-                // cell and position in the cell at level r: exact (power-of-two scaling)
-                const float sr = pow2i(r);
-                const F3 pr = f3(s.pos.x * sr, s.pos.y * sr, s.pos.z * sr);
-                ccx = (uint32_t)pr.x;
-                ccy = (uint32_t)pr.y;
-                ccz = (uint32_t)pr.z;
-                rbp = f3(pr.x - (float)ccx, pr.y - (float)ccy, pr.z - (float)ccz);
-                // the deepest resident node above r holds the brick state
-#pragma unroll 1
-                for (int l = r - 1; l >= 0; --l) {
-                    const uint2 wl = path.w[l * path.stride];
-                    if (wl.x & kResident) {
-                        cur_bw = wl.y;
-                        brick_depth = l;
-                        const float sl = pow2i(l);
-                        const F3 pl = f3(s.pos.x * sl, s.pos.y * sl, s.pos.z * sl);
-                        cur_brp = f3(pl.x - floorf(pl.x), pl.y - floorf(pl.y), pl.z - floorf(pl.z));
-                        break;
-                    }
-                }
-                s.iter += r;
-            }
-        }
-        // ---- descent to the node that stops it
+// The walk of a warp's rays in the unit box; all 32 lanes call it, `alive` the
+// ones that have a ray.
+//
+// The walk is bound by the warp instructions it issues, and left to itself a
+// warp comes apart: lanes that left a loop early ran on alone, at 14 lanes a
+// descent and 5 a brick (256^3 terrain, 512x512).  So the lanes meet by vote
+// before every descent, after it and before every march.  Most segments are
+// descents to an empty constant node and a step to its far side (11 of 15
+// segments of a ray there, 17 of 19 at 2048^3), so lanes that have reached a
+// brick wait until the visitor's kGather of them have, or no lane can go on
+// without, and then march together.  256^3 at 512x512 / 2048^3 at 3840x2160, whole draw:
+// 0.368 / 8.87 ms before; 0.289 / 6.36 ms when every brick is marched at once
+// (kGather 1), 0.280 / 6.20 at 8, 0.287 / 6.15 at 16, 0.315 / 6.65 when every
+// lane is waited for.
+//
+// A position in [0,1) plus one, rounded to zero, holds its first 23 binary
+// digits in the significand: digit 22-d picks the child at depth d (what the
+// shader's repeated doubling of the relative position gives), the common
+// prefix of two positions is the part of the path they share, and a node's
+// lower corner is its position's prefix: all integer operations, one per
+// axis.  Beyond depth 22 (no pool of 10-bit pointers built as a tree reaches
+// 11) the digits come from the scaled position itself.
+// The pool pointer of the deepest resident node of the last descent's path (of
+// the root when there is none), at depth d.
+__device__ __forceinline__ uint32_t brick_pointer(const RaycastParams& p, const PathSlots& path, uint32_t res, int d,
+                                                  uint32_t deep_idx) {
+    const uint32_t i = res == 0u ? 0u : d < kPathLevels ? path.node[d * path.stride] : deep_idx;
+    return __ldg(&p.walk[i].y);
+}
+
+struct NoRefill {
+    static constexpr bool kOn = false;
+    template <class V>
+    __device__ __forceinline__ void take(RayState&, V&, WalkResume&, bool, bool&) {}
+};
+template <int FMT, class V, int AHEAD, bool LIT, bool STAGED, class R>
+__device__ __forceinline__ void walk_warp(const RaycastParams& p, const WalkConsts& k, RayState& s, V& vis,
+                                          const PathSlots& path, bool alive, R&& refill) {
+    constexpr unsigned kAll = 0xFFFFFFFFu;
+    WalkResume wr;
+    uint2 node = k.root;
+    uint32_t deep_idx = 0u;  // the deepest resident node below the levels of the kept path
+    int depth = 0, brick_depth = 0;
+    bool is_const = false, loaded = false;
+    bool pending = false;  // the lane's segment takes samples
+    float t = 0.0f;
+    for (;;) {
         for (;;) {
-            if (++s.iter > k.max_iter) {
-                vis.fail(VV_ERR_TIMEOUT);
-                return false;
-            }
-            if (RESUME && depth < kPathLevels) {
-                path.w[depth * path.stride] = node;
-                path.p[depth * path.stride] = (s.nptr_x << 20) | (s.nptr_y << 10) | s.nptr_z;
-            }
-            is_const = (node.x & kConstant) != 0u;
-            loaded = (node.x & kResident) != 0u;
-            if (loaded) {
-                cur_bw = node.y;
-                cur_brp = rbp;
-                brick_depth = depth;
-            }
-            const uint32_t cx = (node.x >> 20) & 0x3FFu, cy = (node.x >> 10) & 0x3FFu, cz = node.x & 0x3FFu;
-            if ((!is_const && !loaded) || (cx == 0u && cy == 0u && cz == 0u)) break;
-            // ComputeVoxelSize (:429-441) * LodScalar, only when the other two
-            // stop conditions do not decide (it has no side effects), and not
-            // at the levels lodb::clear_range has shown to continue
-            if (depth < skip_lo || depth > skip_hi) {
-                const F3 uh = muls(k.up, vhalf), lh = muls(k.left, vhalf);
-                const F3 ll = normalize3(sub(add(sub(s.pos, uh), lh), k.C));
-                const F3 ur = normalize3(sub(sub(add(s.pos, uh), lh), k.C));
-                const float proj = (1.0f - dot3(ll, ur)) * k.lod;
-                if (k.pixel_size > proj) break;
-            }
-            const F3 boff = muls(rbp, 2.0f);
-            const uint32_t ox = boff.x >= 1.0f ? 1u : 0u;
-            const uint32_t oy = boff.y >= 1.0f ? 1u : 0u;
-            const uint32_t oz = boff.z >= 1.0f ? 1u : 0u;
-            rbp = sub(boff, f3((float)ox, (float)oy, (float)oz));
-            s.nptr_x = cx + ox;
-            s.nptr_y = cy + oy;
-            s.nptr_z = cz + oz;
-            ++depth;
-            if (k.unit_box) {
-                ccx = 2u * ccx + ox;
-                ccy = 2u * ccy + oy;
-                ccz = 2u * ccz + oz;
-            } else {
-                node_size = node_size * 0.5f;
-                ext_min = add(ext_min, muls(f3((float)ox, (float)oy, (float)oz), node_size));
-                ext_max = sub(ext_max, muls(f3(1.0f - (float)ox, 1.0f - (float)oy, 1.0f - (float)oz), node_size));
-            }
-            vhalf = vhalf * 0.5f;
-            node = fetch_node<COUNT>(p, s.nptr_x, s.nptr_y, s.nptr_z, ok);
-            if (!ok) {
-                vis.fail(VV_ERR_BOUNDS);
-                return false;
-            }
-        }
-        if (k.unit_box) {
-            const float sc = pow2i(-depth);
-            ext_min = f3((float)ccx * sc, (float)ccy * sc, (float)ccz * sc);
-            ext_max = f3((float)(ccx + 1u) * sc, (float)(ccy + 1u) * sc, (float)(ccz + 1u) * sc);
-            if (RESUME) {
-                prev_depth = depth;
-                prev_cell = (ccx << 20) | (ccy << 10) | ccz;
-            }
-        }
-        // ---- the leaf segment
-        if (is_const) {
-            const float ratio = pow2i(k.L - depth);
-            const float step = k.RS * ratio;
-            const float aw = (float)(node.y >> 24) / 255.0f;
-            const float t = min_exit(s.pos, s.dir, ext_min, ext_max);
-            const int n = (int)div_step(p, t, step, k.L - depth) + 1;
-            if (aw < 0.005f) {
-                s.pos = add(s.pos, muls(s.dir, (float)n * step));
-            } else {
-                const F3 wstep = muls(s.dir, step);
-                const float sa = 1.0f - pow_pow2(1.0f - aw, k.L - depth);
-                const float4 src = make_float4((float)(node.y & 255u) / 255.0f * ratio,
-                                               (float)((node.y >> 8) & 255u) / 255.0f * ratio,
-                                               (float)((node.y >> 16) & 255u) / 255.0f * ratio, sa);
-#pragma unroll(STEPS)
-                for (int i = 0; i < n; ++i) {
-                    s.pos = add(s.pos, wstep);
-                    if (s.dst.w > k.astop) {
-                        const int rem = n - (i + 1);
-                        s.pos = add(s.pos, muls(s.dir, (float)rem * step));
+            if (refill.kOn) refill.take(s, vis, wr, alive || pending, alive);
+            if (__popc(__ballot_sync(kAll, pending)) >= V::kGather) break;
+            bool go = alive && !pending;
+            if (go) go = alive = vis.segment_begin(s);
+            const unsigned lanes = __ballot_sync(kAll, go);
+            if (lanes == 0u) break;
+            if (go) {
+                int skip_lo = 0, skip_hi = k.L;
+                const lodb::V3 at{s.pos.x, s.pos.y, s.pos.z};
+                if (!lodb::deepest_clears(p.lodk, at)) {
+                    lodb::clear_range(p.lodk, at, skip_lo, skip_hi);
+                    if (skip_hi < skip_lo) skip_lo = skip_hi = 1 << 20;  // none
+                }
+                const uint32_t ix = __float_as_uint(__fadd_rz(s.pos.x, 1.0f)),
+                               iy = __float_as_uint(__fadd_rz(s.pos.y, 1.0f)),
+                               iz = __float_as_uint(__fadd_rz(s.pos.z, 1.0f));
+                uint32_t res = 0u;  // levels of the path whose node is resident
+                uint32_t idx = 0u;  // the node
+                node = k.root;
+                depth = 0;
+                if (wr.prev_depth > 0 && skip_lo == 0) {
+                    // the deepest level whose node holds both this and the last
+                    // position and above which the descent surely continues
+                    const uint32_t diff = (ix ^ wr.ix) | (iy ^ wr.iy) | (iz ^ wr.iz);
+                    const int r = min(min(wr.prev_depth, __clz(diff) - 9), skip_hi + 1);
+                    if (r >= 1 && s.iter + r <= k.max_iter) {
+                        idx = path.node[r * path.stride];
+                        node = __ldg(p.walk + idx);
+                        s.nptr = idx;
+                        depth = r;
+                        s.iter += r;
+                        res = wr.res & ((1u << r) - 1u);
+                    }
+                }
+                // ---- descent to the node that stops it.  The next binary digit
+                // of the position per axis is kept in the top bit of hx, hy, hz.
+                uint32_t hx = ix << (9 + depth), hy = iy << (9 + depth), hz = iz << (9 + depth);
+                const int last = depth + k.max_iter - s.iter;  // depths from here on are past the iteration bound
+                const int first = depth;
+                const unsigned shown = (unsigned)(skip_hi - skip_lo);
+                int error = VV_OK;
+                for (;;) {
+                    if (depth >= last) {
+                        error = VV_ERR_TIMEOUT;
                         break;
                     }
-                    const float T = 1.0f - s.dst.w;
-                    const bool go = vis.sample(kSampleConst, src, s.pos, T, s.nsamples);
-                    s.dst = make_float4(T * src.x + s.dst.x, T * src.y + s.dst.y, T * src.z + s.dst.z,
-                                        T * src.w + s.dst.w);
-                    ++s.nsamples;
-                    if (!go) return false;
+                    if (node.x & kResident) res |= 1u << (depth & 31);
+                    if (depth < kPathLevels) path.node[depth * path.stride] = idx;
+                    else if (node.x & kResident) deep_idx = idx;
+                    const uint32_t link = node.x & kLinkMask;
+                    if (node.x < kConstant || link == 0u) break;  // neither constant nor resident, or no children
+                    // the LOD test, only when the other two stop conditions do
+                    // not decide (it has no side effects), and not at the
+                    // levels lodb::clear_range has shown to continue
+                    if ((unsigned)(depth - skip_lo) > shown && lod_stops(k, s.pos, k.rvh * pow2i(-depth))) break;
+                    if (depth < 23 && link < kLinkOdd) {
+                        // 8 * block + (x | y << 1 | z << 2)
+                        idx = __funnelshift_l(hx, __funnelshift_l(hy, __funnelshift_l(hz, link, 1), 1), 1);
+                    } else if (!odd_child(p, s.pos, depth, idx)) {
+                        error = VV_ERR_BOUNDS;
+                        break;
+                    }
+                    ++depth;
+                    hx += hx;
+                    hy += hy;
+                    hz += hz;
+                    node = __ldg(p.walk + idx);
+                }
+                s.iter += depth - first + 1;
+                if (depth > first) s.nptr = idx;
+                is_const = (node.x & kConstant) != 0u;
+                loaded = (node.x & kResident) != 0u;
+                __syncwarp(lanes);
+                wr.prev_depth = depth < kPathLevels ? depth : 0;
+                wr.ix = ix;
+                wr.iy = iy;
+                wr.iz = iz;
+                wr.res = res;
+                brick_depth = res ? 31 - __clz(res) : 0;
+                t = exit_time(s.pos, s.dir, s.rinv, unit_corner(s.pos, ix, iy, iz, depth), pow2i(-depth));
+                if (error != VV_OK) {
+                    vis.fail(error);
+                    alive = false;
+                } else if (is_const && constant_empty(node.y)) {
+                    step_over_constant(p, k, s, depth, t);
+                    vis.template segment_end<true>(p, s);
+                    // restart from the root (:688-720); the node pointer keeps its value
+                    alive = !(s.dst.w > k.astop) && inside_box(s.pos, k.vmin, k.vmax);
+                } else if (!V::kEverySample && !is_const && p.cell_mask && !(s.dst.w > k.astop) &&
+                           step_over_brick(p, k, s, unit_corner(s.pos, ix, iy, iz, brick_depth),
+                                           brick_pointer(p, path, wr.res, brick_depth, deep_idx), brick_depth, t)) {
+                    vis.template segment_end<true>(p, s);
+                    alive = inside_box(s.pos, k.vmin, k.vmax);
+                } else {
+                    pending = true;
                 }
             }
-        } else {
-            // lightDir = normalize(LightPosition - rayWorldPosition) at entry (:337)
-            const F3 light_dir = LIT ? normalize3(sub(ld3(p.u.light_position), s.pos)) : f3(0.0f, 0.0f, 0.0f);
-            // the six quotients by the pool dimensions from their reciprocals (fixed_div.h)
-            const F3 bptr = f3(fixed_div((float)((cur_bw >> 20) & 0x3FFu), k.pdim.x, p.rpdim[0]),
-                               fixed_div((float)((cur_bw >> 10) & 0x3FFu), k.pdim.y, p.rpdim[1]),
-                               fixed_div((float)(cur_bw & 0x3FFu), k.pdim.z, p.rpdim[2]));
-            const F3 brb = mul(cur_brp, k.bdim);
-            F3 bpos = add(bptr, f3(fixed_div(brb.x, k.pdim.x, p.rpdim[0]), fixed_div(brb.y, k.pdim.y, p.rpdim[1]),
-                                   fixed_div(brb.z, k.pdim.z, p.rpdim[2])));
-            const float ratio = pow2i(k.L - brick_depth);
-            const F3 wstep = muls(muls(s.dir, k.RS), ratio);
-            const float t = min_exit(s.pos, s.dir, ext_min, ext_max);
-            const float step = k.RS * ratio;
-            const int n = (int)div_step(p, t, step, k.L - brick_depth) + 1;
-            // taps inside this brick's slot skip the general texel addressing
-            int base[3] = {(int)((cur_bw >> 20) & 0x3FFu) - 1, (int)((cur_bw >> 10) & 0x3FFu) - 1,
-                           (int)(cur_bw & 0x3FFu) - 1};
-            uint32_t slot_texel0 = 0u, slot_id = kNoSlot;
-            const uint32_t* cmask = nullptr;  // the slot's empty-cell mask (not in footprint counts)
-            if (base[0] >= 0 && base[1] >= 0 && base[2] >= 0 && base[0] % 10 == 0 && base[1] % 10 == 0 &&
-                base[2] % 10 == 0 && base[0] < p.slots[0] * 10 && base[1] < p.slots[1] * 10 &&
-                base[2] < p.slots[2] * 10) {
-                const uint32_t slot = ((uint32_t)base[2] / 10u * (uint32_t)p.slots[1] + (uint32_t)base[1] / 10u) *
-                                          (uint32_t)p.slots[0] + (uint32_t)base[0] / 10u;
-                slot_texel0 = slot * 1000u;
-                slot_id = slot;
-                if (!COUNT && p.cell_mask) cmask = p.cell_mask + (size_t)slot * kCellMaskWords;
-            } else {
-                base[0] = base[1] = base[2] = -100000;
-            }
-            const bool staged = STAGED && stage_acquire(path.stage, p.bricks, slot_id, p.status);
-            const uint32_t* stex = staged ? path.stage->texels : nullptr;
-#pragma unroll(STEPS)
-            for (int i = 0; i < n; ++i) {
-                s.pos = add(s.pos, wstep);
-                if (s.dst.w > k.astop) {
-                    const int rem = n - (i + 1);
-                    s.pos = add(s.pos, muls(s.dir, (float)rem * step));
-                    break;
-                }
-                float4 src;
-                const int in = COUNT ? kOutside : sample_in_slot<FMT, STAGED>(p, bpos, base, slot_texel0, cmask, src, stex);
-                if (in == kOutside) src = sample_brick<FMT, COUNT>(p, bpos);
-                src.w = 1.0f - (1.0f - src.w);
-                // shading adds rgb times finite factors: nothing to a zero sample
-                if (LIT && in != kEmptyCell) light_sample(p, bpos, s.dir, light_dir, src);
-                const float T = 1.0f - s.dst.w;
-                const bool go = vis.sample(kSampleBrick, src, bpos, T, s.nsamples);
-                // a zero sample leaves dst as it is (T * 0 + dst == dst)
-                if (in != kEmptyCell)
-                    s.dst = make_float4(T * src.x + s.dst.x, T * src.y + s.dst.y, T * src.z + s.dst.z,
-                                        T * src.w + s.dst.w);
-                ++s.nsamples;
-                if (!go) {
-                    if (staged) stage_release(path.stage);
-                    return false;
-                }
-                bpos = add(bpos, s.brick_step);
-            }
-            if (staged) stage_release(path.stage);
         }
-        vis.segment_end(s, is_const, loaded);
-        if (s.dst.w > k.astop && (is_const || loaded)) return false;
-        // restart from the root (:688-720); the node pointer keeps its value
-        return inside_box(s.pos, k.vmin, k.vmax);
+        const unsigned bricks = __ballot_sync(kAll, pending && !is_const);
+        if (!__any_sync(kAll, pending)) break;
+        if (pending) {
+            bool go;
+            if (is_const) {
+                go = march_constant(p, k, s, vis, node.y, depth, t);
+            } else {
+                // the position relative to the brick's node, the fractional part of its scaled position
+                const F3 lo = unit_corner(s.pos, wr.ix, wr.iy, wr.iz, brick_depth);
+                BrickMarch b;
+                b.set<false>(p, k, s, brick_pointer(p, path, wr.res, brick_depth, deep_idx), muls(sub(s.pos, lo), pow2i(brick_depth)), brick_depth, t);
+                go = march_brick_warp<FMT, V, AHEAD, LIT, STAGED>(p, k, s, vis, b, bricks, path.stage);
+            }
+            if (go) vis.template segment_end<true>(p, s);
+            alive = go && !(s.dst.w > k.astop && (is_const || loaded)) && inside_box(s.pos, k.vmin, k.vmax);
+            pending = false;
+        }
     }
 }
 
-template <int FMT, bool COUNT, class V, int STEPS = 1, bool RESUME = false, bool LIT = false, bool STAGED = false>
+// walk() runs a ray's segments until its walk has ended; all 32 lanes of a warp
+// call it, `alive` the ones that have a ray.  UNIT: the volume box is [0,1]^3
+// (unit_box), as compute_uniforms makes it; each pixel body keeps the other
+// boxes in a function of its own, out of line, so that they cost the unit box
+// neither registers nor instruction cache.
+template <int FMT, bool COUNT, class V, bool UNIT, int AHEAD, bool LIT = false, bool STAGED = false>
 __device__ __forceinline__ void walk(const RaycastParams& p, const WalkConsts& k, RayState& s, V& vis,
-                                     PathSlots path = PathSlots{nullptr, nullptr, 0, nullptr}) {
-    WalkResume wr;
-    while (walk_segment<FMT, COUNT, V, STEPS, RESUME, LIT, STAGED>(p, k, s, vis, path, wr)) {
+                                     const PathSlots& path, bool alive) {
+    if (UNIT) {
+        walk_warp<FMT, V, AHEAD, LIT, STAGED>(p, k, s, vis, path, alive, NoRefill{});
+    } else if (alive) {
+        while (walk_segment_box<FMT, COUNT, V, LIT>(p, k, s, vis)) {
+        }
     }
 }
 
@@ -895,15 +1278,21 @@ __device__ __forceinline__ void walk(const RaycastParams& p, const WalkConsts& k
 // Entries go straight to the pixel's 12 usage words in memory (zeroed
 // before the walk), which keeps 12 registers free during the walk.
 struct UsageVisitor {
+    static constexpr int kGather = 8;
+    static constexpr bool kEverySample = false;  // samples of empty cells change nothing it records
     uint32_t* out;  // this pixel's usage words, or nullptr
     int list_slot, nl_count, pushed, start_push, max_push;
     int* status;
     __device__ __forceinline__ bool segment_begin(const RayState&) { return true; }
     __device__ __forceinline__ bool sample(int, const float4&, F3, float, int) { return true; }
-    __device__ __forceinline__ void segment_end(const RayState& s, bool, bool) {
+    template <bool UNIT>
+    __device__ __forceinline__ void segment_end(const RaycastParams& p, const RayState& s) {
         if (nl_count >= start_push && nl_count < start_push + 12 && pushed < max_push) {
             ++pushed;
-            const uint32_t bits = ((s.nptr_x + 1u) << 20) | ((s.nptr_y + 1u) << 10) | (s.nptr_z + 1u);
+            uint32_t x, y, z;
+            if (UNIT) node_position(p, s.nptr, x, y, z);
+            else x = s.nptr >> 20, y = (s.nptr >> 10) & 0x3FFu, z = s.nptr & 0x3FFu;
+            const uint32_t bits = ((x + 1u) << 20) | ((y + 1u) << 10) | (z + 1u);
             if (out) out[list_slot] = bits;
             list_slot = list_slot == 11 ? 0 : list_slot + 1;
         }
@@ -946,44 +1335,60 @@ __device__ __forceinline__ void finish_pixel(const RaycastParams& p, size_t pix,
 }
 
 // One pixel of the forward draw: the fragment's ray walk, FragColor and the
-// three RGBA32UI usage-list layers (:490-751).
-template <int FMT, bool COUNT, int STEPS, bool RESUME = false, bool LIT = false, bool STAGED = false>
-__device__ __forceinline__ void render_pixel(const RaycastParams& p, int px, int py,
-                                             PathSlots path = PathSlots{nullptr, nullptr, 0, nullptr}) {
+// three RGBA32UI usage-list layers (:490-751).  All lanes of a warp call it;
+// pixels outside the frame do nothing.
+template <int FMT, bool COUNT, bool UNIT, int AHEAD, bool LIT, bool STAGED>
+__device__ __forceinline__ void pixel_body(const RaycastParams& p, int px, int py, const PathSlots& path) {
+    const bool inside = px < p.u.width && py < p.u.height;
     bool ok = true;
-    const WalkConsts k = walk_consts(p, fetch_node<COUNT>(p, 0, 0, 0, ok));
+    const WalkConsts k = walk_consts(p, UNIT ? __ldg(p.walk) : fetch_node<COUNT>(p, 0, 0, 0, ok));
     UsageVisitor vis;
     RayState s;
-    if (start_pixel(p, k, px, py, s, vis))
-        walk<FMT, COUNT, UsageVisitor, STEPS, RESUME, LIT, STAGED>(p, k, s, vis, path);
-    finish_pixel(p, (size_t)py * p.u.width + px, s);
+    const bool alive = inside && start_pixel(p, k, px, py, s, vis);
+    walk<FMT, COUNT, UsageVisitor, UNIT, AHEAD, LIT, STAGED>(p, k, s, vis, path, alive);
+    if (inside) finish_pixel(p, (size_t)py * p.u.width + px, s);
+}
+template <int FMT, bool LIT>
+__device__ __noinline__ void pixel_body_box(const RaycastParams& p, int px, int py) {
+    pixel_body<FMT, false, false, 1, LIT, false>(p, px, py, PathSlots{nullptr, 0, nullptr});
+}
+template <int FMT, bool COUNT, int AHEAD, bool LIT = false, bool STAGED = false>
+__device__ __forceinline__ void render_pixel(const RaycastParams& p, int px, int py, const PathSlots& path) {
+    if (COUNT) pixel_body<FMT, true, false, 1, LIT, false>(p, px, py, path);
+    else if (unit_box(p.u)) pixel_body<FMT, false, true, AHEAD, LIT, STAGED>(p, px, py, path);
+    else pixel_body_box<FMT, LIT>(p, px, py);
 }
 
 // Persistent ray cast that keeps the lanes of a warp busy: each warp takes
-// 8x4 pixel tiles from a device counter and runs its rays one leaf segment
-// at a time (walk_segment); a lane whose ray has ended takes the next pixel
-// of the warp's tile (ballot + popc rank) before the next segment, instead
-// of idling until the warp's slowest ray ends.  Same pixels, same walk, same
-// results as render_pixel.
-template <int FMT>
-__device__ __forceinline__ void render_refill(const RaycastParams& p, unsigned int* counter, PathSlots path) {
-    const vv_uniforms& u = p.u;
-    const int W = u.width, H = u.height;
-    const int tiles_x = (W + 7) >> 3;
-    const int tiles = tiles_x * ((H + 3) >> 2);
-    const unsigned lane = threadIdx.x & 31u;
-    const unsigned below = (1u << lane) - 1u;
-    bool ok = true;
-    const WalkConsts k = walk_consts(p, fetch_node<false>(p, 0, 0, 0, ok));
-    int tile = 0, taken = 32;  // the warp's tile and how many of its pixels are handed out
-    bool more = true;          // tiles left
-    bool active = false;
-    size_t pix = 0;
-    RayState s;
-    UsageVisitor vis;
-    WalkResume wr;
-    for (;;) {
-        unsigned idle = __ballot_sync(0xFFFFFFFFu, !active);
+// 8x4 pixel tiles from a device counter and walks their rays (walk_warp); a
+// lane whose ray has ended takes the next pixel of the warp's tile (ballot +
+// popc rank) before the next descent, instead of idling until the warp's
+// slowest ray ends.  Same pixels, same walk, same results as render_pixel;
+// volumes in the unit box.
+struct TileRefill {
+    static constexpr bool kOn = true;
+    const RaycastParams& p;
+    const WalkConsts& k;
+    unsigned int* counter;
+    int tiles_x, tiles;
+    int tile, taken;  // the warp's tile and how many of its pixels are handed out
+    bool more;        // tiles left
+    bool has;         // the lane holds pixel `pix`
+    size_t pix;
+    __device__ __forceinline__ TileRefill(const RaycastParams& p_, const WalkConsts& k_, unsigned int* counter_)
+        : p(p_), k(k_), counter(counter_), tile(0), taken(32), more(true), has(false), pix(0) {
+        tiles_x = (p.u.width + 7) >> 3;
+        tiles = tiles_x * ((p.u.height + 3) >> 2);
+    }
+    // All lanes of the warp; busy: the lane's ray goes on.  A lane that is not
+    // finishes its pixel and takes the next one; alive: it has a ray.
+    __device__ __forceinline__ void take(RayState& s, UsageVisitor& vis, WalkResume& wr, bool busy, bool& alive) {
+        const unsigned lane = threadIdx.x & 31u;
+        if (!busy && has) {
+            finish_pixel(p, pix, s);
+            has = false;
+        }
+        unsigned idle = __ballot_sync(0xFFFFFFFFu, !busy);
         while (idle && more) {
             if (taken == 32) {
                 unsigned t = 0u;
@@ -996,26 +1401,29 @@ __device__ __forceinline__ void render_refill(const RaycastParams& p, unsigned i
                 }
             }
             const int n = min(__popc(idle), 32 - taken);
-            const int rank = __popc(idle & below);
-            if (!active && rank < n) {
+            const int rank = __popc(idle & ((1u << lane) - 1u));
+            if (!busy && rank < n) {
                 const int q = taken + rank;
                 const int px = (tile % tiles_x) * 8 + (q & 7), py = (tile / tiles_x) * 4 + (q >> 3);
-                if (px < W && py < H) {
-                    pix = (size_t)py * W + px;
+                if (px < p.u.width && py < p.u.height) {
+                    pix = (size_t)py * p.u.width + px;
                     wr = WalkResume{};
-                    active = start_pixel(p, k, px, py, s, vis);
-                    if (!active) finish_pixel(p, pix, s);
+                    alive = busy = has = start_pixel(p, k, px, py, s, vis);
+                    if (!has) finish_pixel(p, pix, s);
                 }
             }
             taken += n;
-            idle = __ballot_sync(0xFFFFFFFFu, !active);
-        }
-        if (__ballot_sync(0xFFFFFFFFu, active) == 0u) return;
-        if (active && !walk_segment<FMT, false, UsageVisitor, 1, true, false>(p, k, s, vis, path, wr)) {
-            finish_pixel(p, pix, s);
-            active = false;
+            idle = __ballot_sync(0xFFFFFFFFu, !busy);
         }
     }
+};
+template <int FMT>
+__device__ __forceinline__ void render_refill(const RaycastParams& p, unsigned int* counter, const PathSlots& path) {
+    const WalkConsts k = walk_consts(p, __ldg(p.walk));
+    RayState s;
+    UsageVisitor vis;
+    TileRefill refill(p, k, counter);
+    walk_warp<FMT, UsageVisitor, 1, false, false>(p, k, s, vis, path, false, refill);
 }
 
 }  // namespace rc
