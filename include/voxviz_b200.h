@@ -305,9 +305,9 @@ int vv_measure_footprint_views(vv_ctx* ctx, int32_t tree, const vv_uniforms* us,
 
 /* No counterpart in the reference: the adjoint of the ray cast with respect
  * to the brick texels.  vv_render_forward_ckpt runs the ray cast of vv_render
- * (colour only, identical values) and stores per-ray checkpoints (at a leaf
- * segment start every >= 32 composited samples, at most `per_ray` per ray)
- * into `ckpt`, a device buffer of vv_ckpt_bytes(width, height, per_ray)
+ * (colour only, identical values) and stores per-ray checkpoints (records of
+ * the leaf segments that took samples, and past them points to walk from;
+ * at most 2 * `per_ray` records of 24 bytes per ray) into `ckpt`, a device buffer of vv_ckpt_bytes(width, height, per_ray)
  * bytes.  vv_backward then ADDS dL/d(texel) to `grad_texels` (device, one
  * float4 per pool texel, slot-major like the pool) given dL/d(colour)
  * (`dl_dcolor`, device, float4 per pixel) for the same uniforms and pools.

@@ -7,15 +7,18 @@
 // and a brick sample is the trilinear blend of 8 texels, so each texel gets
 // its blend weight times dL/d src_k.  Walking the samples backwards needs
 // T_k, which is not recoverable from the final colour once a sample is
-// opaque, so the forward stores a checkpoint at the start of a leaf segment
-// whenever 32 or more samples were composited since the last one; there the
-// walk restarts from the root, so a checkpoint is only the ray position,
-// dst, the iteration count, the sample index and the node pointer.  The
-// adjoint replays each chunk from its checkpoint (in pieces of at most 64
-// samples, the last piece first), keeps the samples of the piece in local
-// memory and back-propagates through them in reverse.  The control flow
-// (descent, step counts, early termination) is that of the forward and is
-// held fixed, as any reverse-mode derivative of this shader does.
+// opaque, so the forward keeps a record of each leaf segment that took
+// samples: where the ray was and what it had composited (alpha alone: the
+// colour so far enters nothing), which brick or constant, and how many
+// samples.  The adjoint goes through a ray's records from the last to the
+// first, takes a segment's samples again (in pieces of at most 64, the last
+// piece first), keeps the piece in local memory and back-propagates through it
+// in reverse: no descent is repeated.  The last quarter of a ray's records, and
+// all of them outside the unit box, are points to walk from instead (one
+// whenever 32 or more samples were composited since the last), for rays that
+// cross more segments than there are records.  The control flow (descent, step counts, early
+// termination) is that of the forward and is held fixed, as any reverse-mode
+// derivative of this shader does.
 #include "raycast_common.cuh"
 
 namespace vv {
@@ -27,28 +30,70 @@ namespace {
 constexpr int kCkptEvery = 32;
 constexpr int kPiece = 64;
 
+// A record, 24 bytes: the ray's position at the start of the segment and its
+// dst.a there; a brick's pointer or a constant's word, and samples | depth <<
+// 16 | kind << 24 (a walk record: the index of its first sample, and its kind).
 struct Ckpt {
-    float4 a;  // pos.xyz, dst.x
-    float4 b;  // dst.yzw, iter (bits)
-    uint4 c;   // nsamples, nptr
+    float2 p0, p1;
+    uint2 w;
 };
+constexpr int kRecordsPerSlot = 2;  // a caller's record slot has 48 bytes
+enum { kRecBrick = 0, kRecConst = 1, kRecWalk = 2 };
 
 struct CkptVisitor {
     static constexpr int kGather = 8;
     static constexpr bool kEverySample = false;
+    static constexpr bool kRecords = true;
     Ckpt* out;
     int cap, count, last;
+    int segments;  // records of segments there may be; then walk records
     int* status;
-    __device__ __forceinline__ bool segment_begin(const RayState& s) {
-        if ((count == 0 || s.nsamples - last >= kCkptEvery) && count < cap) {
-            Ckpt c;
-            c.a = make_float4(s.pos.x, s.pos.y, s.pos.z, s.dst.x);
-            c.b = make_float4(s.dst.y, s.dst.z, s.dst.w, __int_as_float(s.iter));
-            c.c = make_uint4((uint32_t)s.nsamples, s.nptr, 0u, 0u);
-            out[count++] = c;
+    __device__ __forceinline__ void start(Ckpt* out_, int per_ray, int* status_) {
+        out = out_;
+        cap = per_ray * kRecordsPerSlot;
+        count = 0;
+        last = -kCkptEvery;
+        segments = cap - max(1, cap / 4);
+        status = status_;
+    }
+    __device__ __forceinline__ void put(const RayState& s, uint32_t w0, uint32_t w1) {
+        Ckpt c;
+        c.p0 = make_float2(s.pos.x, s.pos.y);
+        c.p1 = make_float2(s.pos.z, s.dst.w);
+        c.w = make_uint2(w0, w1);
+        out[count] = c;
+    }
+    // (also the box walk's records)
+    __device__ __forceinline__ void box_segment(const RayState& s) {
+        if (s.nsamples - last >= kCkptEvery && count < cap) {
+            put(s, (uint32_t)s.nsamples, (uint32_t)kRecWalk << 24);
+            ++count;
             last = s.nsamples;
         }
-        return true;
+    }
+    __device__ __forceinline__ bool segment_begin(const RayState&) { return true; }
+    // Before and after a segment that may take samples.
+    __device__ __forceinline__ void begin_record(const RayState& s) {
+        if (count < segments) {
+            put(s, 0u, 0u);
+            last = s.nsamples;
+        } else {
+            if (segments >= 0) {  // the first walk record
+                segments = -1;
+                last = s.nsamples - kCkptEvery;
+            }
+            box_segment(s);
+        }
+    }
+    __device__ __forceinline__ void end_record(const RayState& s, int kind, uint32_t word, int depth) {
+        const int n = s.nsamples - last;
+        if (count >= segments || n <= 0) return;
+        if (n > 0xFFFF || depth > 0xFF) {  // does not fit: walked from here on
+            out[count++].w = make_uint2((uint32_t)last, (uint32_t)kRecWalk << 24);
+            segments = -1;
+        } else {
+            out[count++].w = make_uint2(word, (uint32_t)n | ((uint32_t)depth << 16) | ((uint32_t)kind << 24));
+        }
     }
     __device__ __forceinline__ bool sample(int, const float4&, F3, float, int) { return true; }
     template <bool UNIT>
@@ -60,30 +105,38 @@ struct CkptVisitor {
 // sample, negated for a constant-node sample: T > 0 or +0 for brick samples),
 // the sample's alpha, r = dot(dL/dc.rgb, src.rgb) (dL/dc.rgb is constant
 // along the ray) and the brick position.  24 bytes a sample.
-struct ReplayVisitor {
-    static constexpr int kGather = 32;  // without masks to skip by, a march is long: 31.0 ms a fit step, 31.5 at 16
-    static constexpr bool kEverySample = true;  // the gradient scatters empty samples too
-    int first, last, n;
-    float gx, gy, gz;  // dL/dc.rgb
+struct Piece {
     float T[kPiece];
     float a[kPiece];
     float r[kPiece];
     F3 bpos[kPiece];
+    __device__ __forceinline__ void put(int i, int kind, const float4& v, F3 b, float t, float4 g) {
+        T[i] = kind == kSampleBrick ? t : -t;
+        a[i] = v.w;
+        // the first three products of the g.a update, in its order
+        r[i] = g.x * v.x + g.y * v.y + g.z * v.z;
+        bpos[i] = b;
+    }
+};
+// A walk from a point, for the samples [first, last) of the ray.
+struct ReplayVisitor {
+    static constexpr int kGather = 32;
+    static constexpr bool kEverySample = true;  // the gradient scatters empty samples too
+    static constexpr bool kRecords = false;
+    Piece* piece;
+    int first, last, n;
+    float4 g;  // dL/dc
     __device__ __forceinline__ bool segment_begin(const RayState& s) { return s.nsamples < last; }
     __device__ __forceinline__ bool sample(int kind, const float4& v, F3 b, float t, int index) {
-        if (index >= first && n < kPiece) {
-            T[n] = kind == kSampleBrick ? t : -t;
-            a[n] = v.w;
-            // the first three products of the g.a update, in its order
-            r[n] = gx * v.x + gy * v.y + gz * v.z;
-            bpos[n] = b;
-            ++n;
-        }
+        if (index >= first && n < kPiece) piece->put(n++, kind, v, b, t, g);
         return index + 1 < last;
     }
     template <bool UNIT>
     __device__ __forceinline__ void segment_end(const RaycastParams&, const RayState&) {}
     __device__ __forceinline__ void fail(int) {}
+    __device__ __forceinline__ void begin_record(const RayState&) {}
+    __device__ __forceinline__ void end_record(const RayState&, int, uint32_t, int) {}
+    __device__ __forceinline__ void box_segment(const RayState&) {}
 };
 
 // The row of the gradient that holds `slot`: the slot itself (dense), or,
@@ -228,6 +281,28 @@ __device__ __forceinline__ void scatter_texels(const RaycastParams& p, F3 uvw, f
     }
 }
 
+// scatter_texels for a sample of a segment whose slot's gradient row is `row`
+// (-1: none): the taps' cell comes from the segment's slot.  False (and
+// nothing) when the taps leave the slot.
+template <bool F64>
+__device__ __forceinline__ bool scatter_cell(const RaycastParams& p, const SlotView& sv, F3 uvw, float4 d,
+                                             const GradTarget& gt, int row) {
+    const TapCell c(p, sv, uvw);
+    if (!c.in_slot()) return false;
+    if (row < 0) return true;
+    const float fx = c.t[0] - (c.fl[0] - kFloorMagic), fy = c.t[1] - (c.fl[1] - kFloorMagic),
+                fz = c.t[2] - (c.fl[2] - kFloorMagic);
+    const size_t base = (size_t)row * 1000u + (uint32_t)((c.l[2] * 10 + c.l[1]) * 10 + c.l[0]);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int bx = q & 1, by = (q >> 1) & 1, bz = q >> 2;
+        const float w = (bx ? fx : 1.0f - fx) * (by ? fy : 1.0f - fy) * (bz ? fz : 1.0f - fz);
+        if (w == 0.0f) continue;
+        texel_atomic<F64>(gt, base + (uint32_t)(bx + 10 * by + 100 * bz), make_float4(w * d.x, w * d.y, w * d.z, w * d.w));
+    }
+    return true;
+}
+
 __device__ __forceinline__ void pixel_of(int& px, int& py) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     px = blockIdx.x * 16 + (warp & 1) * 8 + (lane & 7);
@@ -254,11 +329,7 @@ __device__ __forceinline__ void forward_pixel(const RaycastParams& p, int px, in
     bool ok = true;
     const WalkConsts k = walk_consts(p, UNIT ? __ldg(p.walk) : fetch_node<false>(p, 0, 0, 0, ok));
     CkptVisitor vis;
-    vis.out = ckpt + pix * (size_t)per_ray;
-    vis.cap = per_ray;
-    vis.count = 0;
-    vis.last = 0;
-    vis.status = p.status;
+    vis.start(ckpt + pix * (size_t)(per_ray * kRecordsPerSlot), per_ray, p.status);
     RayState s;
     s.dst = make_float4(0.f, 0.f, 0.f, 0.f);
     s.nsamples = 0;
@@ -276,9 +347,10 @@ __device__ __noinline__ void forward_pixel_box(const RaycastParams& p, int px, i
 }
 
 // 7 resident CTAs (28 warps) per SM, at most 72 registers per thread: the
-// occupancy that measured fastest for the plain ray cast
+// occupancy that measured fastest for the plain ray cast.  FP32 texels (32
+// registers a sample) take 5: a fit step 18.8 ms against 20.3 at 7, 18.9 at 4.
 template <int FMT>
-__global__ void __launch_bounds__(128, 7) forward_ckpt_kernel(const __grid_constant__ RaycastParams p, int2* hdr,
+__global__ void __launch_bounds__(128, FMT == VV_FMT_FP32 ? 5 : 7) forward_ckpt_kernel(const __grid_constant__ RaycastParams p, int2* hdr,
                                                            Ckpt* ckpt, int per_ray) {
     int px, py;
     pixel_of(px, py);
@@ -290,9 +362,38 @@ __global__ void __launch_bounds__(128, 7) forward_ckpt_kernel(const __grid_const
         forward_pixel_box<FMT>(p, px, py, hdr, ckpt, per_ray);
 }
 
-// One pixel of the adjoint.  F64: binary64 gradient rows; WSUM: the lanes of a
-// cell summed before the atomics (scatter_texels).
-template <int FMT, bool F64, bool WSUM, bool UNIT>
+// The state a walk record restarts from.
+__device__ __forceinline__ RayState walk_state(const RayState& s0, const Ckpt& c) {
+    RayState s = s0;
+    s.pos = f3(c.p0.x, c.p0.y, c.p1.x);
+    s.dst = make_float4(0.f, 0.f, 0.f, c.p1.y);
+    s.iter = 0;  // (the bound on iterations: the forward came through with this part of them)
+    s.nsamples = (int)c.w.x;
+    s.nptr = 0u;
+    return s;
+}
+
+// The piece [first, last) of a ray whose records ran out, walked from its walk
+// record; all lanes of the warp call it, `on` the ones that have such a piece.
+// Out of line: few rays cross more sampled segments than there are records.
+template <int FMT>
+__device__ __noinline__ int replay_tail(const RaycastParams& p, const WalkConsts& k, const RayState& s0, const Ckpt& c,
+                                        Piece* piece, float4 g, int first, int last, bool on, PathSlots path) {
+    ReplayVisitor rv;
+    rv.piece = piece;
+    rv.first = first;
+    rv.last = last;
+    rv.n = 0;
+    rv.g = g;
+    RayState s = walk_state(s0, c);
+    walk<FMT, false, ReplayVisitor, true, 1>(p, k, s, rv, path, on);
+    return rv.n;
+}
+
+// One pixel of the adjoint in the unit box; all lanes of a warp call it.  F64:
+// binary64 gradient rows; WSUM: the lanes of a cell summed before the atomics
+// (scatter_texels).
+template <int FMT, bool F64, bool WSUM>
 __device__ __forceinline__ void backward_pixel(const RaycastParams& p, int px, int py, const int2* hdr,
                                                const Ckpt* ckpt, int per_ray, const float4* dl_dcolor,
                                                const GradTarget& gt, const PathSlots& path) {
@@ -306,81 +407,162 @@ __device__ __forceinline__ void backward_pixel(const RaycastParams& p, int px, i
         g = dl_dcolor[pix];
     }
     const int C = h.x, total = h.y;
-    bool ok = true;
-    const WalkConsts k = walk_consts(p, UNIT ? __ldg(p.walk) : fetch_node<false>(p, 0, 0, 0, ok));
+    const WalkConsts k = walk_consts(p, __ldg(p.walk));
     RayState s0;
-    F3 pos;
+    F3 pos = f3(0.f, 0.f, 0.f);
     bool more = C != 0 && total != 0 && (g.x != 0.f || g.y != 0.f || g.z != 0.f || g.w != 0.f) &&
                 ray_origin(u, k, px, py, pos);
-    if (more) ray_start(p, k, px, py, pos, s0);  // direction of this ray
-    const Ckpt* ck = ckpt + pix * (size_t)per_ray;
+    ray_start(p, k, inside ? px : 0, inside ? py : 0, pos, s0);  // direction of this ray
+    const Ckpt* ck = ckpt + pix * (size_t)(per_ray * kRecordsPerSlot);
     uint32_t c_slot = 0xFFFFFFFFu;  // the last slot scattered into and its gradient row
     int c_row = -1;
-    ReplayVisitor rv;
-    rv.gx = g.x;
-    rv.gy = g.y;
-    rv.gz = g.z;
-    // pieces of the ray's chunks, the last first.  The lanes of a warp take
+    Piece piece;
+    // pieces of the ray's records, the last first.  The lanes of a warp take
     // their pieces together: they meet before every replay and every scatter
     // (left to itself each lane runs ahead on its own, at 8 threads a warp
     // instruction instead of 15).
-    int c = C - 1, m = -1, a = 0, b = total;
+    int c = C - 1, m = -1;
+    int end = total;  // of a walk record's samples
     while (__any_sync(0xFFFFFFFFu, more)) {
-        RayState s = s0;
+        int n = 0;  // samples of the piece
+        bool tail = false;
+        int first = 0, last = 0;
+        Ckpt cc;
+        cc.p0 = cc.p1 = make_float2(0.f, 0.f);
+        cc.w = make_uint2(0u, 0u);
+        BrickMarch b;
+        b.slot_id = kNoSlot;
         if (more) {
-            const Ckpt cc = ck[c];
-            if (m < 0) {
-                a = (int)cc.c.x;
-                m = (b - a - 1) / kPiece;
-            }
-            s.pos = f3(cc.a.x, cc.a.y, cc.a.z);
-            s.dst = make_float4(cc.a.w, cc.b.x, cc.b.y, cc.b.z);
-            s.iter = __float_as_int(cc.b.w);
-            s.nsamples = a;
-            s.nptr = cc.c.y;
-            rv.first = a + m * kPiece;
-            rv.last = min(b, rv.first + kPiece);
-            rv.n = 0;
+            cc = ck[c];
+            tail = (cc.w.y >> 24) == kRecWalk;
+            const int count = tail ? end - (int)cc.w.x : (int)(cc.w.y & 0xFFFFu);
+            if (m < 0) m = (count - 1) / kPiece;
+            first = m * kPiece;
+            last = min(count, first + kPiece);
         }
-        walk<FMT, false, ReplayVisitor, UNIT, 1>(p, k, s, rv, path, more);
+        if (__any_sync(0xFFFFFFFFu, tail)) {  // (copies: the originals stay in registers)
+            const WalkConsts kt = k;
+            const RayState st = s0;
+            const Ckpt ct = cc;
+            n = replay_tail<FMT>(p, kt, st, ct, &piece, g, (int)ct.w.x + first, (int)ct.w.x + last, tail, path);
+        }
+        if (more && !tail) {
+            n = last - first;
+            const int depth = (int)(cc.w.y >> 16) & 255;
+            float da = cc.p1.y;
+            if ((cc.w.y >> 24) == kRecConst) {
+                const float4 src = constant_sample(k, cc.w.x, depth);
+                for (int i = 0; i < last; ++i) {
+                    const float T = 1.0f - da;
+                    if (i >= first) piece.put(i - first, kSampleConst, src, f3(0.f, 0.f, 0.f), T, g);
+                    da = T * src.w + da;
+                }
+            } else {
+                RayState s = s0;
+                s.pos = f3(cc.p0.x, cc.p0.y, cc.p1.x);
+                const F3 lo = unit_corner(s.pos, __float_as_uint(__fadd_rz(s.pos.x, 1.0f)),
+                                          __float_as_uint(__fadd_rz(s.pos.y, 1.0f)),
+                                          __float_as_uint(__fadd_rz(s.pos.z, 1.0f)), depth);
+                b.set<false>(p, k, s, cc.w.x, muls(sub(s.pos, lo), pow2i(depth)), depth, 0.0f);
+                for (int i = 0; i < last; ++i) {
+                    float4 src = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (!b.sv.cmask || sample_needed(p, b.sv, b.bpos)) src = fetch_sample<FMT>(p, b.sv, b.bpos);
+                    src.w = 1.0f - (1.0f - src.w);
+                    const float T = 1.0f - da;
+                    if (i >= first) piece.put(i - first, kSampleBrick, src, b.bpos, T, g);
+                    da = T * src.w + da;
+                    b.bpos = add(b.bpos, b.bstep);
+                }
+            }
+        }
         __syncwarp();
         if (more) {
-            for (int j = rv.n - 1; j >= 0; --j) {
-                const float tj = rv.T[j];
+            if (b.slot_id != kNoSlot && b.slot_id != c_slot) {
+                c_row = grad_row(gt, b.slot_id, p.status);
+                c_slot = b.slot_id;
+            }
+            for (int j = n - 1; j >= 0; --j) {
+                const float tj = piece.T[j];
                 const float t = fabsf(tj);
-                if (!(__float_as_uint(tj) >> 31))
-                    scatter_texels<F64, WSUM>(p, rv.bpos[j], make_float4(g.x * t, g.y * t, g.z * t, g.w * t), gt,
-                                              c_slot, c_row);
+                if (!(__float_as_uint(tj) >> 31)) {
+                    const float4 d = make_float4(g.x * t, g.y * t, g.z * t, g.w * t);
+                    if (WSUM || b.slot_id == kNoSlot || !scatter_cell<F64>(p, b.sv, piece.bpos[j], d, gt, c_row))
+                        scatter_texels<F64, WSUM>(p, piece.bpos[j], d, gt, c_slot, c_row);
+                }
                 // g.a -= dot(g, src), the products summed in the order x, y, z, w
-                g.w = g.w - (rv.r[j] + g.w * rv.a[j]);
+                g.w = g.w - (piece.r[j] + g.w * piece.a[j]);
             }
             if (--m < 0) {
-                b = a;
+                if (tail) end = (int)cc.w.x;
                 more = --c >= 0;
             }
         }
     }
 }
+
+// The same for a volume box other than [0,1]^3: every record is walked from.
 template <int FMT, bool F64, bool WSUM>
 __device__ __noinline__ void backward_pixel_box(const RaycastParams& p, int px, int py, const int2* hdr,
                                                 const Ckpt* ckpt, int per_ray, const float4* dl_dcolor,
                                                 const GradTarget& gt) {
-    backward_pixel<FMT, F64, WSUM, false>(p, px, py, hdr, ckpt, per_ray, dl_dcolor, gt,
-                                          PathSlots{nullptr, 0, nullptr});
+    const vv_uniforms& u = p.u;
+    if (px >= u.width || py >= u.height) return;
+    const size_t pix = (size_t)py * u.width + px;
+    const int2 h = hdr[pix];
+    float4 g = dl_dcolor[pix];
+    if (h.x == 0 || h.y == 0 || (g.x == 0.f && g.y == 0.f && g.z == 0.f && g.w == 0.f)) return;
+    bool ok = true;
+    const WalkConsts k = walk_consts(p, fetch_node<false>(p, 0, 0, 0, ok));
+    RayState s0;
+    F3 pos;
+    if (!ray_origin(u, k, px, py, pos)) return;
+    ray_start(p, k, px, py, pos, s0);
+    const Ckpt* ck = ckpt + pix * (size_t)(per_ray * kRecordsPerSlot);
+    uint32_t c_slot = 0xFFFFFFFFu;
+    int c_row = -1;
+    Piece piece;
+    ReplayVisitor rv;
+    rv.piece = &piece;
+    int b = h.y;
+    for (int c = h.x - 1; c >= 0; --c) {
+        const int a = (int)ck[c].w.x;
+        for (int m = (b - a - 1) / kPiece; m >= 0; --m) {
+            RayState s = walk_state(s0, ck[c]);
+            rv.first = a + m * kPiece;
+            rv.last = min(b, rv.first + kPiece);
+            rv.n = 0;
+            rv.g = g;
+            walk<FMT, false, ReplayVisitor, false, 1>(p, k, s, rv, PathSlots{nullptr, 0, nullptr}, true);
+            for (int j = rv.n - 1; j >= 0; --j) {
+                const float tj = piece.T[j], t = fabsf(tj);
+                if (!(__float_as_uint(tj) >> 31))
+                    scatter_texels<F64, WSUM>(p, piece.bpos[j], make_float4(g.x * t, g.y * t, g.z * t, g.w * t), gt,
+                                              c_slot, c_row);
+                g.w = g.w - (piece.r[j] + g.w * piece.a[j]);
+            }
+        }
+        b = a;
+    }
 }
 
-// 6 resident CTAs per SM (80 registers, fewer spills): on the paged 1080p
-// frames 5.73-5.78 ms against 5.83-6.02 at 7 CTAs and 6.18-6.21 at 8 (the
-// atomics' contention, not the walk's latency, bounds it).
+// 4 resident CTAs per SM (128 registers).  What bounds it is the latency of
+// its loads (texels, and the pieces in local memory) behind a small L1, not
+// warps to switch to: one forward and adjoint of the 1080p frame 6.67 ms at 6
+// CTAs, 6.02 at 5, 5.53 at 4, 5.72 at 3; a fit step of eight 512x512 views of
+// FP32 bricks 27.0, 24.2, 20.2 and 20.0 ms.  Also measured and left: the 8
+// texels of a cell summed in registers along the ray (2.3 times fewer
+// reductions, 7.0 and 23.8 ms: more instructions, and the reductions are not
+// the bound any more), each warp on one block of pixels (5.46, 23.4), each
+// lane starting at another tap (5.71, 22.5), pieces of 32 samples (5.58, 22.1).
 template <int FMT, bool F64, bool WSUM>
-__global__ void __launch_bounds__(128, 6) backward_kernel(const __grid_constant__ RaycastParams p, const int2* hdr,
+__global__ void __launch_bounds__(128, 4) backward_kernel(const __grid_constant__ RaycastParams p, const int2* hdr,
                                                        const Ckpt* ckpt, int per_ray, const float4* dl_dcolor,
                                                        const __grid_constant__ GradTarget gt) {
     int px, py;
     pixel_of_strided(px, py);
     __shared__ uint32_t path[kPathLevels][128];
     if (unit_box(p.u))
-        backward_pixel<FMT, F64, WSUM, true>(p, px, py, hdr, ckpt, per_ray, dl_dcolor, gt,
+        backward_pixel<FMT, F64, WSUM>(p, px, py, hdr, ckpt, per_ray, dl_dcolor, gt,
                                              PathSlots{&path[0][threadIdx.x], 128, nullptr});
     else
         backward_pixel_box<FMT, F64, WSUM>(p, px, py, hdr, ckpt, per_ray, dl_dcolor, gt);
@@ -428,14 +610,20 @@ cudaError_t launch_spread_reduce(const GradTarget& grad, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+namespace {
+// The headers' bytes, rounded up to the records' alignment (an odd number of
+// pixels would leave the 16-byte record vectors on an 8-byte boundary).
+size_t hdr_bytes(int w, int h) { return ((size_t)w * h * sizeof(int2) + 15) / 16 * 16; }
+}  // namespace
+
 size_t ckpt_bytes(int w, int h, int per_ray) {
-    return (size_t)w * h * (sizeof(int2) + (size_t)per_ray * sizeof(Ckpt));
+    return hdr_bytes(w, h) + (size_t)w * h * (size_t)per_ray * kRecordsPerSlot * sizeof(Ckpt);
 }
 
 cudaError_t launch_forward_ckpt(int fmt, const RaycastParams& p, void* ckpt, int per_ray, cudaStream_t s) {
     const int W = p.u.width, H = p.u.height;
     int2* hdr = (int2*)ckpt;
-    Ckpt* ck = (Ckpt*)((char*)ckpt + (size_t)W * H * sizeof(int2));
+    Ckpt* ck = (Ckpt*)((char*)ckpt + hdr_bytes(W, H));
     dim3 block(128), grid((unsigned)((W + 15) / 16), (unsigned)((H + 7) / 8));
     switch (fmt) {
         case VV_FMT_RGBA8: forward_ckpt_kernel<VV_FMT_RGBA8><<<grid, block, 0, s>>>(p, hdr, ck, per_ray); break;
@@ -451,7 +639,7 @@ cudaError_t launch_backward(int fmt, const RaycastParams& p, const void* ckpt, i
                             const GradTarget& grad, cudaStream_t s) {
     const int W = p.u.width, H = p.u.height;
     const int2* hdr = (const int2*)ckpt;
-    const Ckpt* ck = (const Ckpt*)((const char*)ckpt + (size_t)W * H * sizeof(int2));
+    const Ckpt* ck = (const Ckpt*)((const char*)ckpt + hdr_bytes(W, H));
     dim3 block(128), grid((unsigned)((W + 15) / 16), (unsigned)((H + 7) / 8));
 #define VV_BWD(F)                                                                                    \
     if (grad.f64 && grad.warp_sum)                                                                   \

@@ -26,12 +26,13 @@ namespace vv {
 using namespace rc;
 
 // LIT: GigaVoxels.frag with ComputeLighting (gradient pool in p.grads).
-// 7 resident CTAs (28 warps) per SM: at most 72 registers per thread.  The
-// walk is bound by dependency latency, and more warps hide more of it:
-// 1080p paged frames measured 3.74 ms uncapped (82 registers, 5 CTAs),
-// 3.56 ms at 6 CTAs, 3.43 ms at 7 (a few bytes spilled), 3.48 ms at 8.
+// 7 resident CTAs (28 warps) per SM: at most 72 registers per thread.  Whole
+// draws at 4 / 5 / 6 / 7 / 8 CTAs: 2160p over the 2048^3 terrain 7.18 / 6.58 /
+// 6.38 / 6.21 / 6.12 ms, the 256^3 volume at 512x512 0.290 / 0.279 / 0.284 /
+// 0.281 / 0.282 ms, DXT5 there 0.552 / 0.553 / 0.541 / 0.537 / 0.531; lit there
+// 0.381 / 0.386 / 0.386 / 0.396 / 0.399, so lit draws take 5.
 template <int FMT, bool COUNT, bool LIT>
-__global__ void __launch_bounds__(128, 7) raycast_kernel(const __grid_constant__ RaycastParams p) {
+__global__ void __launch_bounds__(128, LIT ? 5 : 7) raycast_kernel(const __grid_constant__ RaycastParams p) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int px = blockIdx.x * 16 + (warp & 1) * 8 + (lane & 7);
     const int py = blockIdx.y * 8 + (warp >> 1) * 4 + (lane >> 3);

@@ -471,6 +471,8 @@ static __device__ __noinline__ bool odd_child(const RaycastParams& p, F3 pos, in
 //                                          before a sample is composited;
 //                                          false ends the walk after it
 //   void segment_end<UNIT>(const RaycastParams&, const RayState&)
+//   void begin_record / end_record, box_segment: around the segments that take
+//                                          samples, for the adjoint's records
 //   void fail(int code)
 // STEPS is the number of samples a march looks ahead (march_brick); the
 // results do not depend on it.
@@ -986,6 +988,13 @@ __device__ __forceinline__ void step_over_constant(const RaycastParams& p, const
     const int n = (int)div_step(p, t, step, k.L - depth) + 1;
     s.pos = add(s.pos, muls(s.dir, (float)n * step));
 }
+// The sample of a constant node.
+__device__ __forceinline__ float4 constant_sample(const WalkConsts& k, uint32_t w1, int depth) {
+    const float ratio = pow2i(k.L - depth);
+    const float aw = (float)(w1 >> 24) / 255.0f;
+    return make_float4((float)(w1 & 255u) / 255.0f * ratio, (float)((w1 >> 8) & 255u) / 255.0f * ratio,
+                       (float)((w1 >> 16) & 255u) / 255.0f * ratio, 1.0f - pow_pow2(1.0f - aw, k.L - depth));
+}
 template <class V>
 __device__ __forceinline__ bool march_constant(const RaycastParams& p, const WalkConsts& k, RayState& s, V& vis,
                                                uint32_t w1, int depth, float t) {
@@ -993,11 +1002,8 @@ __device__ __forceinline__ bool march_constant(const RaycastParams& p, const Wal
     const float step = k.RS * ratio;
     const int n = (int)div_step(p, t, step, k.L - depth) + 1;
     bool go = true;
-    const float aw = (float)(w1 >> 24) / 255.0f;
     const F3 wstep = muls(s.dir, step);
-    const float sa = 1.0f - pow_pow2(1.0f - aw, k.L - depth);
-    const float4 src = make_float4((float)(w1 & 255u) / 255.0f * ratio, (float)((w1 >> 8) & 255u) / 255.0f * ratio,
-                                   (float)((w1 >> 16) & 255u) / 255.0f * ratio, sa);
+    const float4 src = constant_sample(k, w1, depth);
     for (int i = 0; i < n && go; ++i) {
         s.pos = add(s.pos, wstep);
         if (s.dst.w > k.astop) {
@@ -1029,6 +1035,7 @@ __device__ __forceinline__ bool lod_stops(const WalkConsts& k, F3 pos, float vha
 template <int FMT, bool COUNT, class V, bool LIT>
 __device__ __forceinline__ bool walk_segment_box(const RaycastParams& p, const WalkConsts& k, RayState& s, V& vis) {
     if (!vis.segment_begin(s)) return false;
+    vis.box_segment(s);
     bool ok = true;
     uint2 node = k.root;
     F3 ext_min = k.vmin, ext_max = k.vmax;
@@ -1227,11 +1234,15 @@ __device__ __forceinline__ void walk_warp(const RaycastParams& p, const WalkCons
                     vis.template segment_end<true>(p, s);
                     // restart from the root (:688-720); the node pointer keeps its value
                     alive = !(s.dst.w > k.astop) && inside_box(s.pos, k.vmin, k.vmax);
-                } else if (!V::kEverySample && !is_const && p.cell_mask && !(s.dst.w > k.astop) &&
-                           step_over_brick(p, k, s, unit_corner(s.pos, ix, iy, iz, brick_depth),
-                                           brick_pointer(p, path, wr.res, brick_depth, deep_idx), brick_depth, t)) {
-                    vis.template segment_end<true>(p, s);
-                    alive = inside_box(s.pos, k.vmin, k.vmax);
+                } else if (!V::kEverySample && !is_const && p.cell_mask && !(s.dst.w > k.astop)) {
+                    const uint32_t bw = brick_pointer(p, path, wr.res, brick_depth, deep_idx);
+                    if (V::kRecords) vis.begin_record(s);
+                    pending = !step_over_brick(p, k, s, unit_corner(s.pos, ix, iy, iz, brick_depth), bw, brick_depth, t);
+                    if (!pending) {
+                        if (V::kRecords) vis.end_record(s, 0, bw, brick_depth);
+                        vis.template segment_end<true>(p, s);
+                        alive = inside_box(s.pos, k.vmin, k.vmax);
+                    }
                 } else {
                     pending = true;
                 }
@@ -1241,14 +1252,18 @@ __device__ __forceinline__ void walk_warp(const RaycastParams& p, const WalkCons
         if (!__any_sync(kAll, pending)) break;
         if (pending) {
             bool go;
+            if (V::kRecords) vis.begin_record(s);
             if (is_const) {
                 go = march_constant(p, k, s, vis, node.y, depth, t);
+                if (V::kRecords) vis.end_record(s, 1, node.y, depth);
             } else {
                 // the position relative to the brick's node, the fractional part of its scaled position
                 const F3 lo = unit_corner(s.pos, wr.ix, wr.iy, wr.iz, brick_depth);
+                const uint32_t bw = brick_pointer(p, path, wr.res, brick_depth, deep_idx);
                 BrickMarch b;
-                b.set<false>(p, k, s, brick_pointer(p, path, wr.res, brick_depth, deep_idx), muls(sub(s.pos, lo), pow2i(brick_depth)), brick_depth, t);
+                b.set<false>(p, k, s, bw, muls(sub(s.pos, lo), pow2i(brick_depth)), brick_depth, t);
                 go = march_brick_warp<FMT, V, AHEAD, LIT, STAGED>(p, k, s, vis, b, bricks, path.stage);
+                if (V::kRecords) vis.end_record(s, 0, bw, brick_depth);
             }
             if (go) vis.template segment_end<true>(p, s);
             alive = go && !(s.dst.w > k.astop && (is_const || loaded)) && inside_box(s.pos, k.vmin, k.vmax);
@@ -1279,6 +1294,10 @@ __device__ __forceinline__ void walk(const RaycastParams& p, const WalkConsts& k
 // before the walk), which keeps 12 registers free during the walk.
 struct UsageVisitor {
     static constexpr int kGather = 8;
+    static constexpr bool kRecords = false;  // (hooks of the adjoint's records)
+    __device__ __forceinline__ void begin_record(const RayState&) {}
+    __device__ __forceinline__ void end_record(const RayState&, int, uint32_t, int) {}
+    __device__ __forceinline__ void box_segment(const RayState&) {}
     static constexpr bool kEverySample = false;  // samples of empty cells change nothing it records
     uint32_t* out;  // this pixel's usage words, or nullptr
     int list_slot, nl_count, pushed, start_push, max_push;
