@@ -1,7 +1,8 @@
 """The arithmetic of the unit-box walk (voxviz_b200/csrc: fixed_div.h,
-walknode.h, lod_bound.h) against what it stands for, on the host: quotients by
+walknode.h, lod_bound.h, dxt.h) against what it stands for, on the host: quotients by
 a ray's direction equal IEEE division, node records equal the words they are
-made from, and the quick LOD test never clears a level that stops.  The
+made from, the quick LOD test never clears a level that stops, and a DXT5
+texel decoded alone equals its block's.  The
 kernels' bit-exact parity rests on these."""
 import subprocess
 from pathlib import Path
@@ -16,5 +17,5 @@ def test_walk_arithmetic(tmp_path):
     r = subprocess.run([str(exe)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
     counts = [tuple(map(int, line.split())) for line in r.stdout.splitlines()]
-    assert len(counts) == 3 and all(bad == 0 for _, bad in counts)
+    assert len(counts) == 4 and all(bad == 0 for _, bad in counts)
     assert counts[0][0] == 20000000 and counts[1][0] > 2000000 and counts[2][0] > 100000, counts

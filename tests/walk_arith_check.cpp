@@ -1,7 +1,8 @@
 // Host checks of the arithmetic that the unit-box walk takes in place of the
 // shader's own: markstein_div (fixed_div.h) against IEEE division, block_div
 // and walk_link (walknode.h) against their definitions, and
-// lodb::deepest_clears (lod_bound.h) against the exact binary32 LOD test.
+// lodb::deep_levels (lod_bound.h) against the exact binary32 LOD test, and the
+// one-texel DXT5 decode (dxt.h) against the block's.
 // Prints "<checks> <mismatches>" per part; built and run by
 // tests/test_walk_arith.py.
 #include <cmath>
@@ -10,6 +11,7 @@
 #include <cstring>
 #include <random>
 
+#include "../voxviz_b200/csrc/dxt.h"
 #include "../voxviz_b200/csrc/fixed_div.h"
 #include "../voxviz_b200/csrc/lod_bound.h"
 #include "../voxviz_b200/csrc/walknode.h"
@@ -95,18 +97,35 @@ int main() {
         const V3 up = normalize3(cross3(look, left));
         const int L = 3 + (int)(U(rng) * 8);
         const float lod = U(rng) < 0.8f ? 1.0f : 0.25f + 2.f * U(rng);
-        // pixel sizes: any, one ulp above the deepest level's projection (it stops there), below it
-        const float proj = exact_proj(pos, C, up, left, std::ldexp(rvh, -L), lod);
+        // pixel sizes: any, one ulp above a deep level's projection (it stops there), below it
+        const float proj = exact_proj(pos, C, up, left, std::ldexp(rvh, -(L - (int)(it / 3 % 4))), lod);
         const float pix = it % 3 == 0 ? std::pow(10.f, -8.5f + 4.f * U(rng))
                           : it % 3 == 1 ? std::nextafter(proj, 1e30f) : proj * (0.8f + 0.2f * U(rng));
         const vv::lodb::Consts k = vv::lodb::make_consts(C, up, left, rvh, lod, pix, L, true);
-        if (!vv::lodb::deepest_clears(k, pos)) continue;
+        const int hi = vv::lodb::deep_levels(k, pos);
+        if (hi < 0) continue;
         ++checks;
-        for (int l = 0; l <= L; ++l)
+        for (int l = 0; l <= hi; ++l)
             if (pix > exact_proj(pos, C, up, left, std::ldexp(rvh, -l), lod)) {
                 ++bad;
                 break;
             }
+    }
+    std::printf("%ld %ld\n", checks, bad);
+    total_bad += bad;
+    checks = bad = 0;
+    for (uint32_t e = 0; e < 65536u * 8u; ++e) {  // every pair of alpha endpoints and code, colours along
+        const uint32_t a = e & 65535u, code = e >> 16;
+        uint64_t codes = 0;
+        for (int t = 0; t < 16; ++t) codes |= (uint64_t)((code + t) & 7u) << (3 * t);
+        const uint32_t w[4] = {a | (uint32_t)(codes << 16), (uint32_t)(codes >> 16), (uint32_t)rng(), (uint32_t)rng()};
+        for (int t = 0; t < 16; ++t, ++checks)
+            if (vv::dxt::texel_dxt5(w[0], w[1], w[2], w[3], t) != vv::dxt::decode_dxt5(w, t)) ++bad;
+    }
+    for (uint32_t e = 0; e < (1u << 22); ++e, ++checks) {  // colour endpoints
+        const uint32_t w[4] = {(uint32_t)rng(), (uint32_t)rng(), (uint32_t)rng(), (uint32_t)rng()};
+        const int t = (int)(e & 15u);
+        if (vv::dxt::texel_dxt5(w[0], w[1], w[2], w[3], t) != vv::dxt::decode_dxt5(w, t)) ++bad;
     }
     std::printf("%ld %ld\n", checks, bad);
     total_bad += bad;

@@ -82,6 +82,8 @@ VV_HD float scale2(float x, int e) {
 #endif
 }
 
+constexpr int kDeepTries = 3;
+
 // Per-frame constants (made once on the host).
 struct Consts {
     V3 C, w;          // camera position, w = up - left
@@ -95,8 +97,8 @@ struct Consts {
     float rvh;
     int max_level;
     bool ok;
-    // deepest_clears: its level's half voxel size squared and times theta, the
-    // smallest |a|^2 it covers (0 / a huge one: none)
+    // deep_levels: the deepest level's half voxel size squared and times theta,
+    // the smallest |a|^2 it covers (a huge one: none)
     float quick_vh2, quick_theta, quick_min;
 };
 
@@ -134,32 +136,44 @@ VV_HD Consts make_consts(V3 C, V3 up, V3 left, float rvh, float lod, float pixel
     const float s1 = 2.0f * (1.01f * 1.7321f / 0.316f * u + 1.8f * u) * 1.02f;
     const float room = 0.0051f - s1 - 13.2f * u - px * (1.0f + 2e-4f);
     k.ra_shallow = room > 0.0f ? room / s0 * (1.0f - 1e-3f) : 0.0f;
-    // the quick test of the deepest level: |a| at least 4 vh |w| there, and
-    // either no level above j0 or those shown; theta >= 5 Dmax from R >= need
+    // deep_levels: the deepest level's half voxel size vh, and |a| at least
+    // 16 vh' |w| for the size vh' of the highest level tried, so that
+    // vh'^2 |w|^2 / |a|^2 <= 1/256 (and vh' |w| <= |a|/4), and either no level
+    // above j0 or those shown; theta >= 5 Dmax from R >= need
     const float vh = scale2(rvh, -max_level);
-    k.quick_vh2 = 2.0f * vh * vh * (1.0f - 6e-4f);
+    k.quick_vh2 = 2.0f * vh * vh * (1.0f - 2.0f / 256.0f) * (1.0f - 6e-4f);
     k.quick_theta = 1.001f * k.theta * vh;
-    float amin = 4.0f * vh * wn * 40.0f;  // (vh^2 W / A is then below 1/25600)
+    float amin = 16.0f * vh * (float)(1 << (kDeepTries - 1)) * wn;
     if (amin < k.t0) {
         const float shallow = k.ra_shallow > 0.0f ? 1.001f / k.ra_shallow : 1e18f;
         if (amin < shallow) amin = shallow < k.t0 ? shallow : k.t0;
     }
     const float dm = k.d0 / (amin > 1e-6f ? amin : 1e-6f) + k.d1;
-    k.quick_min = k.ok && max_level >= 0 && max_level < 60 && amin > 1e-6f && k.need >= 12.6f * dm * dm
+    k.quick_min = k.ok && max_level >= kDeepTries && max_level < 60 && amin > 1e-6f && k.need >= 12.6f * dm * dm
                       ? amin * amin * 1.001f : 3e38f;
     return k;
 }
 
-// Whether the LOD test surely continues at every level from 0 to max_level:
-// what clear_range shows for the deepest level, with |a| bounded by
-// (1 + |a|^2) / 2 in place of its square root.
-VV_HD bool deepest_clears(const Consts& k, V3 pos) {
+// The deepest level of the last kDeepTries up to which the LOD test surely
+// continues from level 0 on, or -1: clear_range's bound, with |a| bounded by
+// (1 + |a|^2) / 2 in place of its square root (no reciprocals).
+VV_HD int deep_levels(const Consts& k, V3 pos) {
     const V3 a = sub3(pos, k.C);
     const float A = dot(a, a);
     const float aw = dot(a, k.w), AW = A * k.W;
     const float S = AW - aw * aw;
-    return A >= k.quick_min && S >= 0.1002f * AW &&
-           k.quick_vh2 * S >= 1.0005f * A * (k.need * A + k.quick_theta * (k.d0 + k.d1 * (0.5f + 0.5f * A)));
+    if (!(A >= k.quick_min && S >= 0.1002f * AW)) return -1;
+    const float base = 1.0005f * k.need * A * A;
+    float r = k.quick_vh2 * S, d = 1.0005f * A * k.quick_theta * (k.d0 + k.d1 * (0.5f + 0.5f * A));
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+    for (int i = 0; i < kDeepTries; ++i) {
+        if (r >= base + d) return k.max_level - i;
+        r = r * 4.0f;  // the next level up: vh doubled
+        d = d * 2.0f;
+    }
+    return -1;
 }
 
 // Levels [lo, hi] at which the LOD test surely continues for position pos

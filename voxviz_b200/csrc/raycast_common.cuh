@@ -116,16 +116,6 @@ __device__ __forceinline__ void dxt_address(uint32_t i, uint32_t& block, int& t)
 template <>
 struct Texel<VV_FMT_DXT5> {
     static constexpr float kScale = 1.0f / 255.0f;
-    __device__ __forceinline__ static float4 load(const void* pool, uint32_t i) {
-        uint32_t b;
-        int t;
-        dxt_address(i, b, t);
-        const uint4 v = __ldg((const uint4*)pool + b);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-        const uint32_t c = dxt::decode_dxt5(w, t);
-        return make_float4(byte_as_float(c, 0x7440u), byte_as_float(c, 0x7441u), byte_as_float(c, 0x7442u),
-                           byte_as_float(c, 0x7443u));
-    }
 };
 template <>
 struct Texel<VV_FMT_DXT1> {
@@ -210,6 +200,20 @@ struct RawTexel<VV_FMT_RGBA8> {
         const unsigned long long bias = pack2(-8388608.0f, -8388608.0f);
         const Pair4 pa = biased(a), pb = biased(b);
         return Pair4{fma2(tt, sub2(pb.xy, pa.xy), add2(pa.xy, bias)), fma2(tt, sub2(pb.zw, pa.zw), add2(pa.zw, bias))};
+    }
+};
+// DXT5 texels are decoded to RGBA8 words and filtered as those.
+template <>
+struct RawTexel<VV_FMT_DXT5> : RawTexel<VV_FMT_RGBA8> {
+    __device__ __forceinline__ static T decode(const void* pool, uint32_t block, int t) {
+        const uint4 v = __ldg((const uint4*)pool + block);
+        return dxt::texel_dxt5(v.x, v.y, v.z, v.w, t);
+    }
+    __device__ __forceinline__ static T load(const void* pool, uint32_t i) {
+        uint32_t b;
+        int t;
+        dxt_address(i, b, t);
+        return decode(pool, b, t);
     }
 };
 template <int FMT>
@@ -340,6 +344,14 @@ __device__ __forceinline__ float4 fetch_sample(const RaycastParams& p, const Slo
         for (int k = 0; k < 8; ++k) {
             const uint32_t w = stex[l000 + (k & 1) + 10 * ((k >> 1) & 1) + 100 * (k >> 2)];
             memcpy(&v[k], &w, sizeof(w));
+        }
+    } else if constexpr (FMT == VV_FMT_DXT5) {
+        // the taps' blocks from the local texel (4x4 texels of a slice each)
+        const uint32_t blocks = sv.texel0 / 1000u * (uint32_t)dxt::kBlocksPerSlot;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int x = c.l[0] + (k & 1), y = c.l[1] + ((k >> 1) & 1), z = c.l[2] + (k >> 2);
+            v[k] = RawTexel<FMT>::decode(p.bricks, blocks + (uint32_t)dxt::block_of(x, y, z), dxt::texel_of(x, y));
         }
     } else {
         const uint32_t i000 = sv.texel0 + l000;
@@ -1153,9 +1165,10 @@ __device__ __forceinline__ void walk_warp(const RaycastParams& p, const WalkCons
             const unsigned lanes = __ballot_sync(kAll, go);
             if (lanes == 0u) break;
             if (go) {
-                int skip_lo = 0, skip_hi = k.L;
+                int skip_lo = 0, skip_hi;
                 const lodb::V3 at{s.pos.x, s.pos.y, s.pos.z};
-                if (!lodb::deepest_clears(p.lodk, at)) {
+                skip_hi = lodb::deep_levels(p.lodk, at);
+                if (skip_hi < 0) {
                     lodb::clear_range(p.lodk, at, skip_lo, skip_hi);
                     if (skip_hi < skip_lo) skip_lo = skip_hi = 1 << 20;  // none
                 }
