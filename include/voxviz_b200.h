@@ -316,6 +316,10 @@ int vv_measure_footprint_views(vv_ctx* ctx, int32_t tree, const vv_uniforms* us,
 size_t vv_ckpt_bytes(int32_t width, int32_t height, int32_t per_ray);
 int vv_render_forward_ckpt(vv_ctx* ctx, int32_t tree, const vv_uniforms* u, float* color,
                            void* ckpt, int32_t per_ray);
+/* The same for n views of one size in one launch (16 a launch): colours,
+ * checkpoint buffers and dL/d(colour) of the views one after another. */
+int vv_render_forward_ckpt_views(vv_ctx* ctx, int32_t tree, const vv_uniforms* us, int32_t n,
+                                 float* color, void* ckpt, int32_t per_ray);
 int vv_backward(vv_ctx* ctx, int32_t tree, const vv_uniforms* u, const float* dl_dcolor,
                 const void* ckpt, int32_t per_ray, float* grad_texels);
 /* Where vv_backward_ex adds the gradient.  `grad` holds 1000 texels per row,
@@ -360,6 +364,10 @@ typedef struct vv_grad_desc {
 } vv_grad_desc;
 int vv_backward_ex(vv_ctx* ctx, int32_t tree, const vv_uniforms* u, const float* dl_dcolor,
                    const void* ckpt, int32_t per_ray, const vv_grad_desc* g);
+/* vv_backward_ex of n views of one size (see vv_render_forward_ckpt_views). */
+int vv_backward_views(vv_ctx* ctx, int32_t tree, const vv_uniforms* us, int32_t n,
+                      const float* dl_dcolor, const void* ckpt, int32_t per_ray,
+                      const vv_grad_desc* g);
 /* Use caller-owned device memory (e.g. a torch tensor) as the brick pool:
  * slots_x*slots_y*slots_z*1000 texels of `fmt` at `texels`; the context does
  * not free it.  Replaces vv_brickpool_create for differentiable use. */

@@ -445,6 +445,13 @@ class Context:
         self._ck(lib().vv_render_forward_ckpt(self._h, tree, C.byref(u), C.c_void_p(color), C.c_void_p(ckpt),
                                               per_ray), "forward with checkpoints")
 
+    def forward_ckpt_views(self, us: Sequence[Uniforms], color: int, ckpt: int, per_ray: int, tree: int = 0) -> None:
+        """forward_ckpt of views of one size in one launch; colours and
+        checkpoint buffers of the views one after another."""
+        self._ck(lib().vv_render_forward_ckpt_views(self._h, tree, (Uniforms * len(us))(*us), len(us),
+                                                    C.c_void_p(color), C.c_void_p(ckpt), per_ray),
+                 "forward with checkpoints")
+
     def backward(self, u: Uniforms, dl_dcolor: int, ckpt: int, per_ray: int, grad_texels: int,
                  tree: int = 0) -> None:
         self._ck(lib().vv_backward(self._h, tree, C.byref(u), C.c_void_p(dl_dcolor), C.c_void_p(ckpt), per_ray,
@@ -458,12 +465,19 @@ class Context:
         atomics and/or the atomics spread over copies of the rows (binary32
         rows; with `keep` the copies' sums wait for the next spread call
         without it)."""
+        self.backward_views([u], dl_dcolor, ckpt, per_ray, grad, f64, slot_map, rows_used, rows_cap, tree, warp_sum,
+                            spread, keep)
+
+    def backward_views(self, us: Sequence[Uniforms], dl_dcolor: int, ckpt: int, per_ray: int, grad: int,
+                       f64: bool = False, slot_map: int = 0, rows_used: int = 0, rows_cap: int = 0, tree: int = 0,
+                       warp_sum: bool = False, spread: bool = False, keep: bool = False) -> None:
+        """backward_ex of views of one size in one launch (see forward_ckpt_views)."""
         flags = ((N.VV_GRAD_F64 if f64 else 0) | (N.VV_GRAD_WARP_SUM if warp_sum else 0) |
                  (N.VV_GRAD_SPREAD if spread else 0) | (N.VV_GRAD_SPREAD_KEEP if keep else 0))
         g = N.GradDesc(grad=grad, flags=flags, rows_cap=rows_cap, slot_map=slot_map or None,
                        rows_used=rows_used or None)
-        self._ck(lib().vv_backward_ex(self._h, tree, C.byref(u), C.c_void_p(dl_dcolor), C.c_void_p(ckpt), per_ray,
-                                      C.byref(g)), "backward")
+        self._ck(lib().vv_backward_views(self._h, tree, (Uniforms * len(us))(*us), len(us), C.c_void_p(dl_dcolor),
+                                         C.c_void_p(ckpt), per_ray, C.byref(g)), "backward")
 
 
 # --------------------------------------------------------------- batches ---

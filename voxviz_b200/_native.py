@@ -300,8 +300,11 @@ SIGNATURES = {
     "vv_ctx_set_compaction": (C.c_int, [P, C.c_int32]),
     "vv_ckpt_bytes": (C.c_size_t, [C.c_int32, C.c_int32, C.c_int32]),
     "vv_render_forward_ckpt": (C.c_int, [P, C.c_int32, C.POINTER(Uniforms), P, P, C.c_int32]),
+    "vv_render_forward_ckpt_views": (C.c_int, [P, C.c_int32, C.POINTER(Uniforms), C.c_int32, P, P, C.c_int32]),
     "vv_backward": (C.c_int, [P, C.c_int32, C.POINTER(Uniforms), P, P, C.c_int32, P]),
     "vv_backward_ex": (C.c_int, [P, C.c_int32, C.POINTER(Uniforms), P, P, C.c_int32, C.POINTER(GradDesc)]),
+    "vv_backward_views": (C.c_int, [P, C.c_int32, C.POINTER(Uniforms), C.c_int32, P, P, C.c_int32,
+                                    C.POINTER(GradDesc)]),
     "vv_brickpool_attach": (C.c_int, [P, P, C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
     "vv_batch_variants": (C.c_int32, [C.POINTER(BatchConfig), C.c_int32]),
     "vv_render_batch": (C.c_int, [P, C.POINTER(BatchView), C.c_int32, C.POINTER(BatchConfig)]),

@@ -27,6 +27,13 @@ using namespace rc;
 
 namespace {
 
+// The views of a launch: views of one size over the same pools.
+constexpr int kMaxDiffViews = 16;  // 472 bytes each of the launch parameters
+template <int VIEWS>
+struct DiffViews {
+    RaycastParams p[VIEWS];
+};
+
 constexpr int kCkptEvery = 32;
 constexpr int kPiece = 64;
 
@@ -303,20 +310,6 @@ __device__ __forceinline__ bool scatter_cell(const RaycastParams& p, const SlotV
     return true;
 }
 
-__device__ __forceinline__ void pixel_of(int& px, int& py) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    px = blockIdx.x * 16 + (warp & 1) * 8 + (lane & 7);
-    py = blockIdx.y * 8 + (warp >> 1) * 4 + (lane >> 3);
-}
-// The adjoint's pixels: a CTA covers the same 16x8 pixels, each warp every
-// second pixel of them in x and y, so that a warp's lanes sample fewer
-// common texels at once (fewer lanes of one atomic on one address).
-__device__ __forceinline__ void pixel_of_strided(int& px, int& py) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    px = blockIdx.x * 16 + 2 * (lane & 7) + (warp & 1);
-    py = blockIdx.y * 8 + 2 * (lane >> 3) + (warp >> 1);
-}
-
 }  // namespace
 
 // One pixel of the checkpointing forward.
@@ -349,11 +342,15 @@ __device__ __noinline__ void forward_pixel_box(const RaycastParams& p, int px, i
 // 7 resident CTAs (28 warps) per SM, at most 72 registers per thread: the
 // occupancy that measured fastest for the plain ray cast.  FP32 texels (32
 // registers a sample) take 5: a fit step 18.8 ms against 20.3 at 7, 18.9 at 4.
-template <int FMT>
-__global__ void __launch_bounds__(128, FMT == VV_FMT_FP32 ? 5 : 7) forward_ckpt_kernel(const __grid_constant__ RaycastParams p, int2* hdr,
-                                                           Ckpt* ckpt, int per_ray) {
+template <int FMT, int VIEWS, int RAYS>
+__global__ void __launch_bounds__(128, FMT == VV_FMT_FP32 ? 5 : 7)
+    forward_ckpt_kernel(const __grid_constant__ DiffViews<VIEWS> dv, char* ckpts, size_t stride, size_t hdr_size,
+                        int per_ray) {
+    const RaycastParams& p = dv.p[VIEWS > 1 ? blockIdx.z : 0];
+    int2* hdr = (int2*)(ckpts + (VIEWS > 1 ? blockIdx.z * stride : 0));
+    Ckpt* ckpt = (Ckpt*)((char*)hdr + hdr_size);
     int px, py;
-    pixel_of(px, py);
+    warp_pixel<RAYS, false>(px, py);
     __shared__ uint32_t path[kPathLevels][128];
     if (unit_box(p.u))
         forward_pixel<FMT, true>(p, px, py, hdr, ckpt, per_ray,
@@ -554,12 +551,20 @@ __device__ __noinline__ void backward_pixel_box(const RaycastParams& p, int px, 
 // reductions, 7.0 and 23.8 ms: more instructions, and the reductions are not
 // the bound any more), each warp on one block of pixels (5.46, 23.4), each
 // lane starting at another tap (5.71, 22.5), pieces of 32 samples (5.58, 22.1).
-template <int FMT, bool F64, bool WSUM>
-__global__ void __launch_bounds__(128, 4) backward_kernel(const __grid_constant__ RaycastParams p, const int2* hdr,
-                                                       const Ckpt* ckpt, int per_ray, const float4* dl_dcolor,
-                                                       const __grid_constant__ GradTarget gt) {
+//
+// A CTA covers a block of pixels, each warp every second pixel of it in x and
+// y, so that a warp's lanes sample fewer common texels at once (fewer lanes of
+// one atomic on one address).
+template <int FMT, bool F64, bool WSUM, int VIEWS, int RAYS>
+__global__ void __launch_bounds__(128, 4)
+    backward_kernel(const __grid_constant__ DiffViews<VIEWS> dv, const char* ckpts, size_t stride, size_t hdr_size,
+                    int per_ray, const float4* dl, const __grid_constant__ GradTarget gt) {
+    const RaycastParams& p = dv.p[VIEWS > 1 ? blockIdx.z : 0];
+    const int2* hdr = (const int2*)(ckpts + (VIEWS > 1 ? blockIdx.z * stride : 0));
+    const Ckpt* ckpt = (const Ckpt*)((const char*)hdr + hdr_size);
+    const float4* dl_dcolor = dl + (VIEWS > 1 ? (size_t)blockIdx.z * p.u.width * p.u.height : 0);
     int px, py;
-    pixel_of_strided(px, py);
+    warp_pixel<RAYS, true>(px, py);
     __shared__ uint32_t path[kPathLevels][128];
     if (unit_box(p.u))
         backward_pixel<FMT, F64, WSUM>(p, px, py, hdr, ckpt, per_ray, dl_dcolor, gt,
@@ -620,45 +625,107 @@ size_t ckpt_bytes(int w, int h, int per_ray) {
     return hdr_bytes(w, h) + (size_t)w * h * (size_t)per_ray * kRecordsPerSlot * sizeof(Ckpt);
 }
 
-cudaError_t launch_forward_ckpt(int fmt, const RaycastParams& p, void* ckpt, int per_ray, cudaStream_t s) {
-    const int W = p.u.width, H = p.u.height;
-    int2* hdr = (int2*)ckpt;
-    Ckpt* ck = (Ckpt*)((char*)ckpt + hdr_bytes(W, H));
-    dim3 block(128), grid((unsigned)((W + 15) / 16), (unsigned)((H + 7) / 8));
-    switch (fmt) {
-        case VV_FMT_RGBA8: forward_ckpt_kernel<VV_FMT_RGBA8><<<grid, block, 0, s>>>(p, hdr, ck, per_ray); break;
-        case VV_FMT_FP16: forward_ckpt_kernel<VV_FMT_FP16><<<grid, block, 0, s>>>(p, hdr, ck, per_ray); break;
-        case VV_FMT_BF16: forward_ckpt_kernel<VV_FMT_BF16><<<grid, block, 0, s>>>(p, hdr, ck, per_ray); break;
-        case VV_FMT_FP32: forward_ckpt_kernel<VV_FMT_FP32><<<grid, block, 0, s>>>(p, hdr, ck, per_ray); break;
-        default: return cudaErrorInvalidValue;
-    }
+namespace {
+
+// One launch for a call's views, up to kMaxDiffViews: a view of a fit (512x512
+// and less) does not fill the machine, and its slowest rays end alone.
+template <int FMT, int VIEWS>
+cudaError_t forward_views(const RaycastParams* p, int n, char* ckpt, size_t stride, int per_ray, cudaStream_t s) {
+    const int W = p->u.width, H = p->u.height;
+    DiffViews<VIEWS> dv;
+    for (int v = 0; v < n; ++v) dv.p[v] = p[v];
+    const size_t hdr = hdr_bytes(W, H);
+    const int rays = rays_per_warp((long long)n * W * H);
+    const dim3 grid = warp_grid(rays, W, H, n);
+    if (rays == 4) forward_ckpt_kernel<FMT, VIEWS, 4><<<grid, 128, 0, s>>>(dv, ckpt, stride, hdr, per_ray);
+    else if (rays == 16) forward_ckpt_kernel<FMT, VIEWS, 16><<<grid, 128, 0, s>>>(dv, ckpt, stride, hdr, per_ray);
+    else forward_ckpt_kernel<FMT, VIEWS, 32><<<grid, 128, 0, s>>>(dv, ckpt, stride, hdr, per_ray);
     return cudaGetLastError();
 }
 
-cudaError_t launch_backward(int fmt, const RaycastParams& p, const void* ckpt, int per_ray, const float4* dl_dcolor,
-                            const GradTarget& grad, cudaStream_t s) {
-    const int W = p.u.width, H = p.u.height;
-    const int2* hdr = (const int2*)ckpt;
-    const Ckpt* ck = (const Ckpt*)((const char*)ckpt + hdr_bytes(W, H));
-    dim3 block(128), grid((unsigned)((W + 15) / 16), (unsigned)((H + 7) / 8));
-#define VV_BWD(F)                                                                                    \
-    if (grad.f64 && grad.warp_sum)                                                                   \
-        backward_kernel<F, true, true><<<grid, block, 0, s>>>(p, hdr, ck, per_ray, dl_dcolor, grad);   \
-    else if (grad.f64)                                                                               \
-        backward_kernel<F, true, false><<<grid, block, 0, s>>>(p, hdr, ck, per_ray, dl_dcolor, grad);  \
-    else if (grad.warp_sum)                                                                          \
-        backward_kernel<F, false, true><<<grid, block, 0, s>>>(p, hdr, ck, per_ray, dl_dcolor, grad);  \
-    else                                                                                             \
-        backward_kernel<F, false, false><<<grid, block, 0, s>>>(p, hdr, ck, per_ray, dl_dcolor, grad);
+template <int FMT, bool F64, bool WSUM, int VIEWS>
+cudaError_t backward_views(const RaycastParams* p, int n, const char* ckpt, size_t stride, int per_ray,
+                           const float4* dl, const GradTarget& gt, cudaStream_t s) {
+    const int W = p->u.width, H = p->u.height;
+    DiffViews<VIEWS> dv;
+    for (int v = 0; v < n; ++v) dv.p[v] = p[v];
+    const size_t hdr = hdr_bytes(W, H);
+    // (the forms for checks and comparisons take full warps)
+    const int rays = F64 || WSUM ? 32 : rays_per_warp((long long)n * W * H);
+    const dim3 grid = warp_grid(rays, W, H, n);
+    if constexpr (!F64 && !WSUM) {
+        if (rays == 4) {
+            backward_kernel<FMT, F64, WSUM, VIEWS, 4><<<grid, 128, 0, s>>>(dv, ckpt, stride, hdr, per_ray, dl, gt);
+            return cudaGetLastError();
+        }
+        if (rays == 16) {
+            backward_kernel<FMT, F64, WSUM, VIEWS, 16><<<grid, 128, 0, s>>>(dv, ckpt, stride, hdr, per_ray, dl, gt);
+            return cudaGetLastError();
+        }
+    }
+    backward_kernel<FMT, F64, WSUM, VIEWS, 32><<<grid, 128, 0, s>>>(dv, ckpt, stride, hdr, per_ray, dl, gt);
+    return cudaGetLastError();
+}
+
+template <int FMT>
+cudaError_t backward_form(const RaycastParams* p, int n, const char* ckpt, size_t stride, int per_ray, const float4* dl,
+                          const GradTarget& gt, cudaStream_t s) {
+    const size_t npix = (size_t)p->u.width * p->u.height;
+    cudaError_t e = cudaSuccess;
+    for (int v = 0; v < n && e == cudaSuccess; v += kMaxDiffViews) {
+        const int m = n - v < kMaxDiffViews ? n - v : kMaxDiffViews;
+        if (m > 1 && !gt.f64 && !gt.warp_sum) {
+            e = backward_views<FMT, false, false, kMaxDiffViews>(p + v, m, ckpt + (size_t)v * stride, stride, per_ray,
+                                                                 dl + (size_t)v * npix, gt, s);
+            continue;
+        }
+        for (int i = v; i < v + m && e == cudaSuccess; ++i) {
+            const char* ck = ckpt + (size_t)i * stride;
+            const float4* d = dl + (size_t)i * npix;
+            if (gt.f64 && gt.warp_sum) e = backward_views<FMT, true, true, 1>(p + i, 1, ck, stride, per_ray, d, gt, s);
+            else if (gt.f64) e = backward_views<FMT, true, false, 1>(p + i, 1, ck, stride, per_ray, d, gt, s);
+            else if (gt.warp_sum) e = backward_views<FMT, false, true, 1>(p + i, 1, ck, stride, per_ray, d, gt, s);
+            else e = backward_views<FMT, false, false, 1>(p + i, 1, ck, stride, per_ray, d, gt, s);
+        }
+    }
+    return e;
+}
+
+template <int FMT>
+cudaError_t forward_form(const RaycastParams* p, int n, char* ckpt, size_t stride, int per_ray, cudaStream_t s) {
+    cudaError_t e = cudaSuccess;
+    for (int v = 0; v < n && e == cudaSuccess; v += kMaxDiffViews) {
+        const int m = n - v < kMaxDiffViews ? n - v : kMaxDiffViews;
+        char* ck = ckpt + (size_t)v * stride;
+        e = m > 1 ? forward_views<FMT, kMaxDiffViews>(p + v, m, ck, stride, per_ray, s)
+                  : forward_views<FMT, 1>(p + v, 1, ck, stride, per_ray, s);
+    }
+    return e;
+}
+
+}  // namespace
+
+cudaError_t launch_forward_ckpt(int fmt, const RaycastParams* p, int n, void* ckpt, size_t stride, int per_ray,
+                                cudaStream_t s) {
     switch (fmt) {
-        case VV_FMT_RGBA8: VV_BWD(VV_FMT_RGBA8) break;
-        case VV_FMT_FP16: VV_BWD(VV_FMT_FP16) break;
-        case VV_FMT_BF16: VV_BWD(VV_FMT_BF16) break;
-        case VV_FMT_FP32: VV_BWD(VV_FMT_FP32) break;
+        case VV_FMT_RGBA8: return forward_form<VV_FMT_RGBA8>(p, n, (char*)ckpt, stride, per_ray, s);
+        case VV_FMT_FP16: return forward_form<VV_FMT_FP16>(p, n, (char*)ckpt, stride, per_ray, s);
+        case VV_FMT_BF16: return forward_form<VV_FMT_BF16>(p, n, (char*)ckpt, stride, per_ray, s);
+        case VV_FMT_FP32: return forward_form<VV_FMT_FP32>(p, n, (char*)ckpt, stride, per_ray, s);
         default: return cudaErrorInvalidValue;
     }
-#undef VV_BWD
-    return cudaGetLastError();
+}
+
+cudaError_t launch_backward(int fmt, const RaycastParams* p, int n, const void* ckpt, size_t stride, int per_ray,
+                            const float4* dl_dcolor, const GradTarget& grad, cudaStream_t s) {
+    const char* ck = (const char*)ckpt;
+    switch (fmt) {
+        case VV_FMT_RGBA8: return backward_form<VV_FMT_RGBA8>(p, n, ck, stride, per_ray, dl_dcolor, grad, s);
+        case VV_FMT_FP16: return backward_form<VV_FMT_FP16>(p, n, ck, stride, per_ray, dl_dcolor, grad, s);
+        case VV_FMT_BF16: return backward_form<VV_FMT_BF16>(p, n, ck, stride, per_ray, dl_dcolor, grad, s);
+        case VV_FMT_FP32: return backward_form<VV_FMT_FP32>(p, n, ck, stride, per_ray, dl_dcolor, grad, s);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 }  // namespace vv

@@ -492,16 +492,36 @@ static int diff_params(vv_ctx* c, int32_t tree, const vv_uniforms* u, RaycastPar
     return VV_OK;
 }
 
-int vv_render_forward_ckpt(vv_ctx* c, int32_t tree, const vv_uniforms* u, float* color, void* ckpt,
-                           int32_t per_ray) {
-    RaycastParams p;
-    int rc = diff_params(c, tree, u, p);
+// The launch parameters of a call's views, which have one size.
+static int diff_views(vv_ctx* c, int32_t tree, const vv_uniforms* us, int32_t n, std::vector<RaycastParams>& p) {
+    if (!us || n <= 0) return fail(c, VV_ERR_ARG, "bad arguments");
+    p.resize((size_t)n);
+    for (int32_t v = 0; v < n; ++v) {
+        const int rc = diff_params(c, tree, us + v, p[(size_t)v]);
+        if (rc) return rc;
+        if (us[v].width != us[0].width || us[v].height != us[0].height)
+            return fail(c, VV_ERR_ARG, "the views of a call must have one size");
+    }
+    return VV_OK;
+}
+
+int vv_render_forward_ckpt_views(vv_ctx* c, int32_t tree, const vv_uniforms* us, int32_t n, float* color, void* ckpt,
+                                 int32_t per_ray) {
+    std::vector<RaycastParams> p;
+    int rc = diff_views(c, tree, us, n, p);
     if (rc) return rc;
     if (!ckpt || per_ray <= 0) return fail(c, VV_ERR_ARG, "checkpoint buffer required");
     cudaSetDevice(c->device);
-    p.color = (float4*)color;
-    VV_CUDA(c, launch_forward_ckpt(c->fmt, p, ckpt, per_ray, c->stream));
+    const size_t npix = (size_t)us->width * us->height;
+    for (int32_t v = 0; v < n; ++v) p[(size_t)v].color = color ? (float4*)color + (size_t)v * npix : nullptr;
+    VV_CUDA(c, launch_forward_ckpt(c->fmt, p.data(), n, ckpt, ckpt_bytes(us->width, us->height, per_ray), per_ray,
+                                   c->stream));
     return VV_OK;
+}
+
+int vv_render_forward_ckpt(vv_ctx* c, int32_t tree, const vv_uniforms* u, float* color, void* ckpt,
+                           int32_t per_ray) {
+    return vv_render_forward_ckpt_views(c, tree, u, 1, color, ckpt, per_ray);
 }
 
 int vv_backward(vv_ctx* c, int32_t tree, const vv_uniforms* u, const float* dl_dcolor, const void* ckpt,
@@ -514,8 +534,13 @@ int vv_backward(vv_ctx* c, int32_t tree, const vv_uniforms* u, const float* dl_d
 
 int vv_backward_ex(vv_ctx* c, int32_t tree, const vv_uniforms* u, const float* dl_dcolor, const void* ckpt,
                    int32_t per_ray, const vv_grad_desc* g) {
-    RaycastParams p;
-    int rc = diff_params(c, tree, u, p);
+    return vv_backward_views(c, tree, u, 1, dl_dcolor, ckpt, per_ray, g);
+}
+
+int vv_backward_views(vv_ctx* c, int32_t tree, const vv_uniforms* us, int32_t n, const float* dl_dcolor,
+                      const void* ckpt, int32_t per_ray, const vv_grad_desc* g) {
+    std::vector<RaycastParams> p;
+    int rc = diff_views(c, tree, us, n, p);
     if (rc) return rc;
     if (!ckpt || per_ray <= 0 || !dl_dcolor || !g || !g->grad) return fail(c, VV_ERR_ARG, "bad backward buffers");
     if ((g->flags & ~(VV_GRAD_F64 | VV_GRAD_WARP_SUM | VV_GRAD_SPREAD | VV_GRAD_SPREAD_KEEP)) != 0)
@@ -565,7 +590,8 @@ int vv_backward_ex(vv_ctx* c, int32_t tree, const vv_uniforms* u, const float* d
         gt.spread = c->d_spread;
         gt.spread_rows = (int)rows;
     }
-    VV_CUDA(c, launch_backward(c->fmt, p, ckpt, per_ray, (const float4*)dl_dcolor, gt, c->stream));
+    VV_CUDA(c, launch_backward(c->fmt, p.data(), n, ckpt, ckpt_bytes(us->width, us->height, per_ray), per_ray,
+                               (const float4*)dl_dcolor, gt, c->stream));
     if (keep) {
         c->spread_rows_kept = gt.spread_rows;
     } else {

@@ -31,11 +31,10 @@ using namespace rc;
 // 6.38 / 6.21 / 6.12 ms, the 256^3 volume at 512x512 0.290 / 0.279 / 0.284 /
 // 0.281 / 0.282 ms, DXT5 there 0.552 / 0.553 / 0.541 / 0.537 / 0.531; lit there
 // 0.381 / 0.386 / 0.386 / 0.396 / 0.399, so lit draws take 5.
-template <int FMT, bool COUNT, bool LIT>
+template <int FMT, bool COUNT, bool LIT, int RAYS>
 __global__ void __launch_bounds__(128, LIT ? 5 : 7) raycast_kernel(const __grid_constant__ RaycastParams p) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int px = blockIdx.x * 16 + (warp & 1) * 8 + (lane & 7);
-    const int py = blockIdx.y * 8 + (warp >> 1) * 4 + (lane >> 3);
+    int px, py;
+    warp_pixel<RAYS, false>(px, py);
     __shared__ uint32_t path[kPathLevels][128];
     render_pixel<FMT, COUNT, 1, LIT>(p, px, py, PathSlots{&path[0][threadIdx.x], 128, nullptr});
 }
@@ -116,15 +115,25 @@ cudaError_t launch_raycast_refill(int fmt, const RaycastParams& p, unsigned int*
     return cudaGetLastError();
 }
 
+namespace {
+template <int FMT, bool LIT>
+void launch_rays(const RaycastParams& p, cudaStream_t s) {
+    const int rays = rays_per_warp((long long)p.u.width * p.u.height);
+    const dim3 grid = warp_grid(rays, p.u.width, p.u.height);
+    if (rays == 4) raycast_kernel<FMT, false, LIT, 4><<<grid, 128, 0, s>>>(p);
+    else if (rays == 16) raycast_kernel<FMT, false, LIT, 16><<<grid, 128, 0, s>>>(p);
+    else raycast_kernel<FMT, false, LIT, 32><<<grid, 128, 0, s>>>(p);
+}
+}  // namespace
+
 cudaError_t launch_raycast(int fmt, const RaycastParams& p, cudaStream_t s) {
-    dim3 block(128);
-    dim3 grid((unsigned)((p.u.width + 15) / 16), (unsigned)((p.u.height + 7) / 8));
     const bool count = p.node_touch && p.brick_touch;
     const bool lit = p.u.compute_lighting && p.grads && !count;
-#define VV_LAUNCH(F)                                                           \
-    if (count) raycast_kernel<F, true, false><<<grid, block, 0, s>>>(p);       \
-    else if (lit) raycast_kernel<F, false, true><<<grid, block, 0, s>>>(p);    \
-    else raycast_kernel<F, false, false><<<grid, block, 0, s>>>(p);
+    const dim3 grid = warp_grid(32, p.u.width, p.u.height);
+#define VV_LAUNCH(F)                                                                \
+    if (count) raycast_kernel<F, true, false, 32><<<grid, 128, 0, s>>>(p);          \
+    else if (lit) launch_rays<F, true>(p, s);                                       \
+    else launch_rays<F, false>(p, s);
     switch (fmt) {
         case VV_FMT_RGBA8: VV_LAUNCH(VV_FMT_RGBA8) break;
         case VV_FMT_FP16: VV_LAUNCH(VV_FMT_FP16) break;

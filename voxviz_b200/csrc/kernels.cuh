@@ -91,7 +91,10 @@ cudaError_t launch_raycast_refill(int fmt, const RaycastParams& p, unsigned int*
 cudaError_t launch_raycast_staged(int fmt, const RaycastParams& p, cudaStream_t s);
 // Differentiable forward (colour + per-ray checkpoints) and its adjoint.
 size_t ckpt_bytes(int w, int h, int per_ray);
-cudaError_t launch_forward_ckpt(int fmt, const RaycastParams& p, void* ckpt, int per_ray, cudaStream_t s);
+// n views of one size over the same pools; view v's checkpoints at ckpt + v *
+// stride, its dL/d(colour) after the view before's.
+cudaError_t launch_forward_ckpt(int fmt, const RaycastParams* p, int n, void* ckpt, size_t stride, int per_ray,
+                                cudaStream_t s);
 // Where the adjoint adds dL/d(texel): `grad` holds 4 floats (or, with f64,
 // 4 doubles) per texel, 1000 texels per row; row = brick-pool slot (dense,
 // slot_map NULL) or the row the slot map assigns (claimed on first touch
@@ -112,8 +115,8 @@ struct GradTarget {
     float4* spread;   // copies 1..copies-1
     int spread_rows;  // rows per copy
 };
-cudaError_t launch_backward(int fmt, const RaycastParams& p, const void* ckpt, int per_ray, const float4* dl_dcolor,
-                            const GradTarget& grad, cudaStream_t s);
+cudaError_t launch_backward(int fmt, const RaycastParams* p, int n, const void* ckpt, size_t stride, int per_ray,
+                            const float4* dl_dcolor, const GradTarget& grad, cudaStream_t s);
 cudaError_t launch_spread_reduce(const GradTarget& grad, cudaStream_t s);
 cudaError_t launch_select(const uint4* usage, uint32_t* mask, uint32_t* level0, int w, int h,
                           cudaStream_t s);

@@ -1391,6 +1391,36 @@ __device__ __forceinline__ void render_pixel(const RaycastParams& p, int px, int
     else pixel_body_box<FMT, LIT>(p, px, py);
 }
 
+// The pixel of a thread of a 128-thread CTA whose warps take RAYS pixels each
+// (warp_tile_w x warp_tile_h; lanes past them get a pixel outside any frame).
+// STRIDED: each warp has every second pixel of the CTA's block in x and y.
+//
+// A launch with few rays leaves most schedulers without a warp while one warp
+// serves the different paths of 32 rays; its time is that of its slowest warp.
+// With fewer rays a warp each path is shorter and the machine fuller (ray cast
+// alone, us, 96x64 of the 128^3 / 256^3 / 1024^3 terrain: 132 / 190 / 212 with
+// 32 rays, 113 / 124 / 188 with 16, 101 / 120 / 179 with 8, 91 / 105 / 140 with
+// 4; 160x120: 117 / 205 / 312, 115 / 154 / 252, 109 / 152 / 230, 106 / 135 /
+// 199; 256x192: 140 / 202 / 298, 124 / 169 / 263, 140 / 212 / 273, 155 / 220 /
+// 260; 384x288: 156 / 232 / 308, 149 / 195 / 306, 189 / 278 / 335; 512x512:
+// 174 / 292 / 336, 213 / 292 / 346), until the warps are more than the
+// machine holds: the lines of rays_per_warp.
+__host__ __device__ constexpr int warp_tile_w(int rays) { return rays == 32 ? 8 : rays == 16 ? 4 : 2; }
+__host__ __device__ constexpr int warp_tile_h(int rays) { return rays == 32 ? 4 : rays == 16 ? 4 : 2; }
+inline int rays_per_warp(long long rays) { return rays <= 24576 ? 4 : rays <= 114688 ? 16 : 32; }
+template <int RAYS, bool STRIDED>
+__device__ __forceinline__ void warp_pixel(int& px, int& py) {
+    constexpr int w = warp_tile_w(RAYS), h = warp_tile_h(RAYS);
+    const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
+    px = blockIdx.x * (2 * w) + (STRIDED ? 2 * (lane % w) + (warp & 1) : (warp & 1) * w + lane % w);
+    py = blockIdx.y * (2 * h) + (STRIDED ? 2 * (lane / w) + (warp >> 1) : (warp >> 1) * h + lane / w);
+    if (RAYS < 32 && lane >= RAYS) px = 1 << 24;
+}
+inline dim3 warp_grid(int rays, int width, int height, int views = 1) {
+    const int w = 2 * warp_tile_w(rays), h = 2 * warp_tile_h(rays);
+    return dim3((unsigned)((width + w - 1) / w), (unsigned)((height + h - 1) / h), (unsigned)views);
+}
+
 // Persistent ray cast that keeps the lanes of a warp busy: each warp takes
 // 8x4 pixel tiles from a device counter and walks their rays (walk_warp); a
 // lane whose ray has ended takes the next pixel of the warp's tile (ballot +

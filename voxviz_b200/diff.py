@@ -85,8 +85,7 @@ class RayCast(torch.autograd.Function):
         color = torch.empty((V, H, W, 4), dtype=torch.float32, device=pool.device)
         nb = Context.ckpt_bytes(W, H, per_ray)
         ckpt = torch.empty((V, nb), dtype=torch.uint8, device=pool.device)
-        for v, u in enumerate(uniforms):
-            ctx.forward_ckpt(u, color[v].data_ptr(), ckpt[v].data_ptr(), per_ray)
+        ctx.forward_ckpt_views(uniforms, color.data_ptr(), ckpt.data_ptr(), per_ray)
         fctx.vctx = ctx
         fctx.slots = slots
         fctx.uniforms = list(uniforms)
@@ -103,10 +102,8 @@ class RayCast(torch.autograd.Function):
         _bind_stream(ctx, pool.device)
         g = grad_color.contiguous().to(torch.float32)
         grad = torch.zeros_like(pool)
-        last = len(fctx.uniforms) - 1
-        for v, u in enumerate(fctx.uniforms):
-            ctx.backward_ex(u, g[v].data_ptr(), ckpt[v].data_ptr(), fctx.per_ray, grad.data_ptr(),
-                            spread=fctx.spread, keep=fctx.spread and v < last)
+        ctx.backward_views(fctx.uniforms, g.data_ptr(), ckpt.data_ptr(), fctx.per_ray, grad.data_ptr(),
+                           spread=fctx.spread)
         return grad, None, None, None, None, None
 
 
