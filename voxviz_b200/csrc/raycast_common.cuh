@@ -455,6 +455,12 @@ __device__ __forceinline__ void node_position(const RaycastParams& p, uint32_t i
     z = 2u * bz + ((i >> 2) & 1u);
 }
 
+// Index of the child in block `link` by the top bit of each axis' digits:
+// 8 * block + (x | y << 1 | z << 2).
+__device__ __forceinline__ uint32_t child_index(uint32_t link, uint32_t hx, uint32_t hy, uint32_t hz) {
+    return __funnelshift_l(hx, __funnelshift_l(hy, __funnelshift_l(hz, link, 1), 1), 1);
+}
+
 // The child of node `idx` at `depth` that holds pos, into idx, where the
 // walk's record does not give it (walknode.h: an odd or bad pointer) or the
 // position's fixed-point digits have run out; false out of the grid.
@@ -594,17 +600,18 @@ __device__ __forceinline__ bool ray_start(const RaycastParams& p, const WalkCons
     return inside_box(s.pos, k.vmin, k.vmax);
 }
 
-// The path of the ray's last descent, per thread in shared memory: the index
-// of the node of each level, `stride` elements apart per level.  A later
-// descent whose position lies in the same level-r node, and whose LOD test
-// lodb::clear_range shows to continue at every level above r, starts at that
-// node instead of the root: the levels it skips would take exactly the
-// recorded path (same nodes, every stop condition false), so the walk is
-// unchanged.
+// The path of the ray's last descent, per thread in shared memory: the child
+// link (walknode.h) of the node of each level it went on from, `stride`
+// elements apart per level.  A later descent whose position lies in the same
+// level-r node, and whose LOD test lodb::clear_range shows to continue at
+// every level down to r, starts at that node's child: the levels it skips
+// would take exactly the recorded path (same nodes, every stop condition
+// false), so the walk is unchanged.  (Starting at node r itself, by its index,
+// cost one more dependent load and visit of three a segment.)
 constexpr int kPathLevels = 11;  // levels 0..10
 struct StageBuf;
 struct PathSlots {
-    uint32_t* node;
+    uint32_t* link;
     int stride;
     StageBuf* stage;  // the warp's staged brick (VV_RAYCAST_STAGED), else nullptr
 };
@@ -1132,12 +1139,15 @@ struct WalkResume {
 // lower corner is its position's prefix: all integer operations, one per
 // axis.  Beyond depth 22 (no pool of 10-bit pointers built as a tree reaches
 // 11) the digits come from the scaled position itself.
-// The pool pointer of the deepest resident node of the last descent's path (of
-// the root when there is none), at depth d.
-__device__ __forceinline__ uint32_t brick_pointer(const RaycastParams& p, const PathSlots& path, uint32_t res, int d,
-                                                  uint32_t deep_idx) {
-    const uint32_t i = res == 0u ? 0u : d < kPathLevels ? path.node[d * path.stride] : deep_idx;
-    return __ldg(&p.walk[i].y);
+// The pool pointer of the deepest resident node (at depth d) of the last
+// descent, whose position the resume state holds.
+constexpr uint32_t kOnPath = 0xFFFFFFFFu;
+__device__ __forceinline__ uint32_t brick_pointer(const RaycastParams& p, const PathSlots& path, const WalkResume& wr,
+                                                  int d, uint32_t brick_idx) {
+    if (brick_idx == kOnPath)
+        brick_idx = d == 0 ? 0u : child_index(path.link[(d - 1) * path.stride], wr.ix << (8 + d), wr.iy << (8 + d),
+                                              wr.iz << (8 + d));
+    return __ldg(&p.walk[brick_idx].y);
 }
 
 struct NoRefill {
@@ -1151,7 +1161,7 @@ __device__ __forceinline__ void walk_warp(const RaycastParams& p, const WalkCons
     constexpr unsigned kAll = 0xFFFFFFFFu;
     WalkResume wr;
     uint2 node = k.root;
-    uint32_t deep_idx = 0u;  // the deepest resident node below the levels of the kept path
+    uint32_t brick_idx = 0u;  // the deepest resident node of the path, or kOnPath: by the kept path
     int depth = 0, brick_depth = 0;
     bool is_const = false, loaded = false;
     bool pending = false;  // the lane's segment takes samples
@@ -1179,18 +1189,20 @@ __device__ __forceinline__ void walk_warp(const RaycastParams& p, const WalkCons
                 uint32_t idx = 0u;  // the node
                 node = k.root;
                 depth = 0;
+                brick_idx = 0u;
                 if (wr.prev_depth > 0 && skip_lo == 0) {
-                    // the deepest level whose node holds both this and the last
-                    // position and above which the descent surely continues
+                    // the deepest node the last descent went on from that holds
+                    // this position too and from which this one surely goes on
                     const uint32_t diff = (ix ^ wr.ix) | (iy ^ wr.iy) | (iz ^ wr.iz);
-                    const int r = min(min(wr.prev_depth, __clz(diff) - 9), skip_hi + 1);
-                    if (r >= 1 && s.iter + r <= k.max_iter) {
-                        idx = path.node[r * path.stride];
+                    const int r = min(min(wr.prev_depth - 1, __clz(diff) - 9), skip_hi);
+                    if (r >= 0 && s.iter + r + 1 <= k.max_iter) {
+                        depth = r + 1;
+                        idx = child_index(path.link[r * path.stride], ix << (9 + r), iy << (9 + r), iz << (9 + r));
                         node = __ldg(p.walk + idx);
                         s.nptr = idx;
-                        depth = r;
-                        s.iter += r;
-                        res = wr.res & ((1u << r) - 1u);
+                        s.iter += depth;
+                        res = wr.res & ((2u << r) - 1u);
+                        brick_idx = res ? kOnPath : 0u;
                     }
                 }
                 // ---- descent to the node that stops it.  The next binary digit
@@ -1200,26 +1212,31 @@ __device__ __forceinline__ void walk_warp(const RaycastParams& p, const WalkCons
                 const int first = depth;
                 const unsigned shown = (unsigned)(skip_hi - skip_lo);
                 int error = VV_OK;
+                bool odd = false;  // a child that its link does not give: no path to resume
                 for (;;) {
                     if (depth >= last) {
                         error = VV_ERR_TIMEOUT;
                         break;
                     }
-                    if (node.x & kResident) res |= 1u << (depth & 31);
-                    if (depth < kPathLevels) path.node[depth * path.stride] = idx;
-                    else if (node.x & kResident) deep_idx = idx;
+                    if (node.x & kResident) {
+                        res |= 1u << (depth & 31);
+                        brick_idx = idx;
+                    }
                     const uint32_t link = node.x & kLinkMask;
                     if (node.x < kConstant || link == 0u) break;  // neither constant nor resident, or no children
                     // the LOD test, only when the other two stop conditions do
                     // not decide (it has no side effects), and not at the
                     // levels lodb::clear_range has shown to continue
                     if ((unsigned)(depth - skip_lo) > shown && lod_stops(k, s.pos, k.rvh * pow2i(-depth))) break;
+                    if (depth < kPathLevels) path.link[depth * path.stride] = link;
                     if (depth < 23 && link < kLinkOdd) {
-                        // 8 * block + (x | y << 1 | z << 2)
-                        idx = __funnelshift_l(hx, __funnelshift_l(hy, __funnelshift_l(hz, link, 1), 1), 1);
-                    } else if (!odd_child(p, s.pos, depth, idx)) {
-                        error = VV_ERR_BOUNDS;
-                        break;
+                        idx = child_index(link, hx, hy, hz);
+                    } else {
+                        odd = true;
+                        if (!odd_child(p, s.pos, depth, idx)) {
+                            error = VV_ERR_BOUNDS;
+                            break;
+                        }
                     }
                     ++depth;
                     hx += hx;
@@ -1232,7 +1249,7 @@ __device__ __forceinline__ void walk_warp(const RaycastParams& p, const WalkCons
                 is_const = (node.x & kConstant) != 0u;
                 loaded = (node.x & kResident) != 0u;
                 __syncwarp(lanes);
-                wr.prev_depth = depth < kPathLevels ? depth : 0;
+                wr.prev_depth = depth < kPathLevels && !odd ? depth : 0;
                 wr.ix = ix;
                 wr.iy = iy;
                 wr.iz = iz;
@@ -1248,7 +1265,7 @@ __device__ __forceinline__ void walk_warp(const RaycastParams& p, const WalkCons
                     // restart from the root (:688-720); the node pointer keeps its value
                     alive = !(s.dst.w > k.astop) && inside_box(s.pos, k.vmin, k.vmax);
                 } else if (!V::kEverySample && !is_const && p.cell_mask && !(s.dst.w > k.astop)) {
-                    const uint32_t bw = brick_pointer(p, path, wr.res, brick_depth, deep_idx);
+                    const uint32_t bw = brick_pointer(p, path, wr, brick_depth, brick_idx);
                     if (V::kRecords) vis.begin_record(s);
                     pending = !step_over_brick(p, k, s, unit_corner(s.pos, ix, iy, iz, brick_depth), bw, brick_depth, t);
                     if (!pending) {
@@ -1272,7 +1289,7 @@ __device__ __forceinline__ void walk_warp(const RaycastParams& p, const WalkCons
             } else {
                 // the position relative to the brick's node, the fractional part of its scaled position
                 const F3 lo = unit_corner(s.pos, wr.ix, wr.iy, wr.iz, brick_depth);
-                const uint32_t bw = brick_pointer(p, path, wr.res, brick_depth, deep_idx);
+                const uint32_t bw = brick_pointer(p, path, wr, brick_depth, brick_idx);
                 BrickMarch b;
                 b.set<false>(p, k, s, bw, muls(sub(s.pos, lo), pow2i(brick_depth)), brick_depth, t);
                 go = march_brick_warp<FMT, V, AHEAD, LIT, STAGED>(p, k, s, vis, b, bricks, path.stage);
