@@ -1165,11 +1165,13 @@ __device__ __forceinline__ void walk_warp(const RaycastParams& p, const WalkCons
     int depth = 0, brick_depth = 0;
     bool is_const = false, loaded = false;
     bool pending = false;  // the lane's segment takes samples
+    // lanes to wait for, of the rays the warp has
+    const int gather = refill.kOn ? V::kGather : max(1, V::kGather * __popc(__ballot_sync(kAll, alive)) / 32);
     float t = 0.0f;
     for (;;) {
         for (;;) {
             if (refill.kOn) refill.take(s, vis, wr, alive || pending, alive);
-            if (__popc(__ballot_sync(kAll, pending)) >= V::kGather) break;
+            if (__popc(__ballot_sync(kAll, pending)) >= gather) break;
             bool go = alive && !pending;
             if (go) go = alive = vis.segment_begin(s);
             const unsigned lanes = __ballot_sync(kAll, go);
