@@ -300,9 +300,12 @@ __device__ __forceinline__ bool scatter_cell(const RaycastParams& p, const SlotV
     const float fx = c.t[0] - (c.fl[0] - kFloorMagic), fy = c.t[1] - (c.fl[1] - kFloorMagic),
                 fz = c.t[2] - (c.fl[2] - kFloorMagic);
     const size_t base = (size_t)row * 1000u + (uint32_t)((c.l[2] * 10 + c.l[1]) * 10 + c.l[0]);
+    const int lane = (int)(threadIdx.x & 31u);
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-        const int bx = q & 1, by = (q >> 1) & 1, bz = q >> 2;
+        // each lane starts at another tap: fewer lanes of one instruction on one texel
+        const int tap = (q + lane) & 7;
+        const int bx = tap & 1, by = (tap >> 1) & 1, bz = tap >> 2;
         const float w = (bx ? fx : 1.0f - fx) * (by ? fy : 1.0f - fy) * (bz ? fz : 1.0f - fz);
         if (w == 0.0f) continue;
         texel_atomic<F64>(gt, base + (uint32_t)(bx + 10 * by + 100 * bz), make_float4(w * d.x, w * d.y, w * d.z, w * d.w));
@@ -350,7 +353,7 @@ __global__ void __launch_bounds__(128, FMT == VV_FMT_FP32 ? 5 : 7)
     int2* hdr = (int2*)(ckpts + (VIEWS > 1 ? blockIdx.z * stride : 0));
     Ckpt* ckpt = (Ckpt*)((char*)hdr + hdr_size);
     int px, py;
-    warp_pixel<RAYS, false>(px, py);
+    warp_pixel<RAYS>(px, py);
     __shared__ uint32_t path[kPathLevels][128];
     if (unit_box(p.u))
         forward_pixel<FMT, true>(p, px, py, hdr, ckpt, per_ray,
@@ -549,12 +552,17 @@ __device__ __noinline__ void backward_pixel_box(const RaycastParams& p, int px, 
 // FP32 bricks 27.0, 24.2, 20.2 and 20.0 ms.  Also measured and left: the 8
 // texels of a cell summed in registers along the ray (2.3 times fewer
 // reductions, 7.0 and 23.8 ms: more instructions, and the reductions are not
-// the bound any more), each warp on one block of pixels (5.46, 23.4), each
-// lane starting at another tap (5.71, 22.5), pieces of 32 samples (5.58, 22.1).
+// the bound any more), pieces of 32 samples (5.58, 22.1), two samples' texels
+// in flight together (0.98-1.00 of the speed), positions summed again instead
+// of kept (1.02 and 0.87 of it).
 //
-// A CTA covers a block of pixels, each warp every second pixel of it in x and
-// y, so that a warp's lanes sample fewer common texels at once (fewer lanes of
-// one atomic on one address).
+// Each warp has a block of pixels of its own and each lane starts at another
+// tap.  Close to the terrain, where thousands of samples fall on one texel, the
+// reductions' contention is the bound: backward of two such 1080p views (34445
+// and 14119 bricks touched) 16.8 and 9.7 ms with neither, 12.2 and 7.8 with the
+// taps alone, 14.4 and 9.1 with the blocks alone, 10.2 and 7.1 with both; the
+// usual views (5.3 and 4.9) take 4.6 and 4.0 with the blocks, 4.8 and 4.3 with
+// both; fit steps are within 4 %.
 template <int FMT, bool F64, bool WSUM, int VIEWS, int RAYS>
 __global__ void __launch_bounds__(128, 4)
     backward_kernel(const __grid_constant__ DiffViews<VIEWS> dv, const char* ckpts, size_t stride, size_t hdr_size,
@@ -564,7 +572,7 @@ __global__ void __launch_bounds__(128, 4)
     const Ckpt* ckpt = (const Ckpt*)((const char*)hdr + hdr_size);
     const float4* dl_dcolor = dl + (VIEWS > 1 ? (size_t)blockIdx.z * p.u.width * p.u.height : 0);
     int px, py;
-    warp_pixel<RAYS, true>(px, py);
+    warp_pixel<RAYS>(px, py);
     __shared__ uint32_t path[kPathLevels][128];
     if (unit_box(p.u))
         backward_pixel<FMT, F64, WSUM>(p, px, py, hdr, ckpt, per_ray, dl_dcolor, gt,

@@ -34,7 +34,7 @@ using namespace rc;
 template <int FMT, bool COUNT, bool LIT, int RAYS>
 __global__ void __launch_bounds__(128, LIT ? 5 : 7) raycast_kernel(const __grid_constant__ RaycastParams p) {
     int px, py;
-    warp_pixel<RAYS, false>(px, py);
+    warp_pixel<RAYS>(px, py);
     __shared__ uint32_t path[kPathLevels][128];
     render_pixel<FMT, COUNT, 1, LIT>(p, px, py, PathSlots{&path[0][threadIdx.x], 128, nullptr});
 }

@@ -1412,7 +1412,6 @@ __device__ __forceinline__ void render_pixel(const RaycastParams& p, int px, int
 
 // The pixel of a thread of a 128-thread CTA whose warps take RAYS pixels each
 // (warp_tile_w x warp_tile_h; lanes past them get a pixel outside any frame).
-// STRIDED: each warp has every second pixel of the CTA's block in x and y.
 //
 // A launch with few rays leaves most schedulers without a warp while one warp
 // serves the different paths of 32 rays; its time is that of its slowest warp.
@@ -1427,12 +1426,12 @@ __device__ __forceinline__ void render_pixel(const RaycastParams& p, int px, int
 __host__ __device__ constexpr int warp_tile_w(int rays) { return rays == 32 ? 8 : rays == 16 ? 4 : 2; }
 __host__ __device__ constexpr int warp_tile_h(int rays) { return rays == 32 ? 4 : rays == 16 ? 4 : 2; }
 inline int rays_per_warp(long long rays) { return rays <= 24576 ? 4 : rays <= 114688 ? 16 : 32; }
-template <int RAYS, bool STRIDED>
+template <int RAYS>
 __device__ __forceinline__ void warp_pixel(int& px, int& py) {
     constexpr int w = warp_tile_w(RAYS), h = warp_tile_h(RAYS);
     const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
-    px = blockIdx.x * (2 * w) + (STRIDED ? 2 * (lane % w) + (warp & 1) : (warp & 1) * w + lane % w);
-    py = blockIdx.y * (2 * h) + (STRIDED ? 2 * (lane / w) + (warp >> 1) : (warp >> 1) * h + lane / w);
+    px = blockIdx.x * (2 * w) + (warp & 1) * w + lane % w;
+    py = blockIdx.y * (2 * h) + (warp >> 1) * h + lane / w;
     if (RAYS < 32 && lane >= RAYS) px = 1 << 24;
 }
 inline dim3 warp_grid(int rays, int width, int height, int views = 1) {
