@@ -3,6 +3,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -494,8 +495,12 @@ static int diff_params(vv_ctx* c, int32_t tree, const vv_uniforms* u, RaycastPar
 
 // The launch parameters of a call's views, which have one size.
 static int diff_views(vv_ctx* c, int32_t tree, const vv_uniforms* us, int32_t n, std::vector<RaycastParams>& p) {
-    if (!us || n <= 0) return fail(c, VV_ERR_ARG, "bad arguments");
-    p.resize((size_t)n);
+    if (!us || n <= 0 || n > 65536) return fail(c, VV_ERR_ARG, "bad arguments");
+    try {
+        p.resize((size_t)n);
+    } catch (const std::bad_alloc&) {
+        return fail(c, VV_ERR_OOM, "launch parameters");
+    }
     for (int32_t v = 0; v < n; ++v) {
         const int rc = diff_params(c, tree, us + v, p[(size_t)v]);
         if (rc) return rc;
