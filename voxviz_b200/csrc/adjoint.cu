@@ -486,16 +486,20 @@ __device__ __forceinline__ void backward_pixel(const RaycastParams& p, int px, i
         }
         __syncwarp();
         if (more) {
-            if (b.slot_id != kNoSlot && b.slot_id != c_slot) {
-                c_row = grad_row(gt, b.slot_id, p.status);
+            // the segment's row, its own: scatter_texels moves (c_slot, c_row) to
+            // the slot of a sample that left the segment's
+            int row = -1;
+            if (b.slot_id != kNoSlot) {
+                row = b.slot_id == c_slot ? c_row : grad_row(gt, b.slot_id, p.status);
                 c_slot = b.slot_id;
+                c_row = row;
             }
             for (int j = n - 1; j >= 0; --j) {
                 const float tj = piece.T[j];
                 const float t = fabsf(tj);
                 if (!(__float_as_uint(tj) >> 31)) {
                     const float4 d = make_float4(g.x * t, g.y * t, g.z * t, g.w * t);
-                    if (WSUM || b.slot_id == kNoSlot || !scatter_cell<F64>(p, b.sv, piece.bpos[j], d, gt, c_row))
+                    if (WSUM || b.slot_id == kNoSlot || !scatter_cell<F64>(p, b.sv, piece.bpos[j], d, gt, row))
                         scatter_texels<F64, WSUM>(p, piece.bpos[j], d, gt, c_slot, c_row);
                 }
                 // g.a -= dot(g, src), the products summed in the order x, y, z, w
