@@ -475,11 +475,14 @@ __device__ __forceinline__ void backward_pixel(const RaycastParams& p, int px, i
                 b.set<false>(p, k, s, cc.w.x, muls(sub(s.pos, lo), pow2i(depth)), depth, 0.0f);
                 for (int i = 0; i < last; ++i) {
                     float4 src = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (!b.sv.cmask || sample_needed(p, b.sv, b.bpos)) src = fetch_sample<FMT>(p, b.sv, b.bpos);
-                    src.w = 1.0f - (1.0f - src.w);
                     const float T = 1.0f - da;
+                    // (an empty sample leaves the alpha as it is, also where T is infinite)
+                    if (!b.sv.cmask || sample_needed(p, b.sv, b.bpos)) {
+                        src = fetch_sample<FMT>(p, b.sv, b.bpos);
+                        src.w = 1.0f - (1.0f - src.w);
+                        da = T * src.w + da;
+                    }
                     if (i >= first) piece.put(i - first, kSampleBrick, src, b.bpos, T, g);
-                    da = T * src.w + da;
                     b.bpos = add(b.bpos, b.bstep);
                 }
             }

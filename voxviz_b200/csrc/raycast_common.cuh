@@ -887,14 +887,17 @@ template <bool LIT>
 __device__ __forceinline__ F3 entry_light(const RaycastParams& p, const RayState& s) {
     return LIT ? normalize3(sub(ld3(p.u.light_position), s.pos)) : f3(0.0f, 0.0f, 0.0f);
 }
-// One sample composited; false when the visitor ends the walk after it.
+// One sample composited (the zero of an empty cell only counted: T * 0 + dst is
+// dst but for an infinite T, and lighting adds nothing to it); false when the
+// visitor ends the walk after it.
 template <bool LIT, class V>
-__device__ __forceinline__ bool take_sample(const RaycastParams& p, RayState& s, V& vis, float4 src, F3 bpos, F3 light_dir) {
+__device__ __forceinline__ bool take_sample(const RaycastParams& p, RayState& s, V& vis, float4 src, F3 bpos, F3 light_dir,
+                                            bool empty) {
     src.w = 1.0f - (1.0f - src.w);
-    if (LIT) light_sample(p, bpos, s.dir, light_dir, src);
+    if (LIT && !empty) light_sample(p, bpos, s.dir, light_dir, src);
     const float T = 1.0f - s.dst.w;
     const bool go = vis.sample(kSampleBrick, src, bpos, T, s.nsamples);
-    s.dst = composite(T, src, s.dst);
+    if (!empty) s.dst = composite(T, src, s.dst);
     ++s.nsamples;
     return go;
 }
@@ -911,7 +914,7 @@ __device__ __forceinline__ bool march_brick(const RaycastParams& p, const WalkCo
             break;
         }
         const float4 src = COUNT ? sample_brick<FMT, COUNT>(p, b.bpos) : fetch_sample<FMT>(p, b.sv, b.bpos);
-        go = take_sample<LIT>(p, s, vis, src, b.bpos, light_dir);
+        go = take_sample<LIT>(p, s, vis, src, b.bpos, light_dir, false);
         b.bpos = add(b.bpos, b.bstep);
     }
     return go;
@@ -981,9 +984,9 @@ __device__ __forceinline__ bool march_brick_warp(const RaycastParams& p, const W
         if (need) {
             s.pos = add(s.pos, b.wstep);
             float4 src = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (!V::kEverySample || !b.sv.cmask || sample_needed(p, b.sv, b.bpos))
-                src = fetch_sample<FMT, STAGED>(p, b.sv, b.bpos, stex);
-            go = take_sample<LIT>(p, s, vis, src, b.bpos, light_dir);
+            const bool empty = V::kEverySample && b.sv.cmask && !sample_needed(p, b.sv, b.bpos);
+            if (!empty) src = fetch_sample<FMT, STAGED>(p, b.sv, b.bpos, stex);
+            go = take_sample<LIT>(p, s, vis, src, b.bpos, light_dir, empty);
             b.bpos = add(b.bpos, b.bstep);
             --left;
             if (left > 0 && s.dst.w > k.astop) {  // the step at which the stop is seen, then the rest at once
