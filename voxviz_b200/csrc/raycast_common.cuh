@@ -1140,8 +1140,8 @@ struct WalkResume {
 // shader's repeated doubling of the relative position gives), the common
 // prefix of two positions is the part of the path they share, and a node's
 // lower corner is its position's prefix: all integer operations, one per
-// axis.  Beyond depth 22 (no pool of 10-bit pointers built as a tree reaches
-// 11) the digits come from the scaled position itself.
+// axis.  Beyond depth 22 (a chain of nodes takes one block a level, so a pool
+// may hold one of any depth) the digits come from the scaled position itself.
 // The pool pointer of the deepest resident node (at depth d) of the last
 // descent, whose position the resume state holds.
 constexpr uint32_t kOnPath = 0xFFFFFFFFu;
@@ -1218,6 +1218,7 @@ __device__ __forceinline__ void walk_warp(const RaycastParams& p, const WalkCons
                 const unsigned shown = (unsigned)(skip_hi - skip_lo);
                 int error = VV_OK;
                 bool odd = false;  // a child that its link does not give: no path to resume
+                int deep = 0;      // the last resident level past the 32 of res, but for the last node's
                 for (;;) {
                     if (depth >= last) {
                         error = VV_ERR_TIMEOUT;
@@ -1238,6 +1239,7 @@ __device__ __forceinline__ void walk_warp(const RaycastParams& p, const WalkCons
                         idx = child_index(link, hx, hy, hz);
                     } else {
                         odd = true;
+                        if (depth > 31 && (node.x & kResident)) deep = depth;
                         if (!odd_child(p, s.pos, depth, idx)) {
                             error = VV_ERR_BOUNDS;
                             break;
@@ -1259,7 +1261,8 @@ __device__ __forceinline__ void walk_warp(const RaycastParams& p, const WalkCons
                 wr.iy = iy;
                 wr.iz = iz;
                 wr.res = res;
-                brick_depth = res ? 31 - __clz(res) : 0;
+                // (levels past 31 share the bits of res: a chain of nodes may be that deep)
+                brick_depth = loaded ? depth : max(deep, 31 - __clz(res));  // (deep is 0 without one)
                 t = exit_time(s.pos, s.dir, s.rinv, unit_corner(s.pos, ix, iy, iz, depth), pow2i(-depth));
                 if (error != VV_OK) {
                     vis.fail(error);
