@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(128, FMT == VV_FMT_FP32 ? 5 : 7)
     int px, py;
     warp_pixel<RAYS>(px, py);
     __shared__ uint32_t path[kPathLevels][128];
-    if (unit_box(p.u))
+    if (unit_walk(p))
         forward_pixel<FMT, true>(p, px, py, hdr, ckpt, per_ray,
                                  PathSlots{&path[0][threadIdx.x], 128, nullptr});
     else
@@ -705,7 +705,7 @@ cudaError_t backward_views(const RaycastParams* p, int n, const char* ckpt, size
 template <int FMT, bool F64, bool WSUM>
 cudaError_t backward_view(const RaycastParams* p, const char* ckpt, size_t stride, int per_ray, const float4* dl,
                           const GradTarget& gt, cudaStream_t s) {
-    if (is_unit_box(p->u)) return backward_views<FMT, F64, WSUM, 1>(p, 1, ckpt, stride, per_ray, dl, gt, s);
+    if (takes_unit_walk(*p)) return backward_views<FMT, F64, WSUM, 1>(p, 1, ckpt, stride, per_ray, dl, gt, s);
     const int W = p->u.width, H = p->u.height;
     backward_box_kernel<FMT, F64, WSUM><<<warp_grid(32, W, H), 128, 0, s>>>(*p, ckpt, hdr_bytes(W, H), per_ray, dl, gt);
     return cudaGetLastError();
@@ -719,7 +719,7 @@ cudaError_t backward_form(const RaycastParams* p, int n, const char* ckpt, size_
     for (int v = 0; v < n && e == cudaSuccess; v += kMaxDiffViews) {
         const int m = n - v < kMaxDiffViews ? n - v : kMaxDiffViews;
         bool unit = true;
-        for (int i = v; i < v + m; ++i) unit = unit && is_unit_box(p[i].u);
+        for (int i = v; i < v + m; ++i) unit = unit && takes_unit_walk(p[i]);
         if (m > 1 && unit && !gt.f64 && !gt.warp_sum) {
             e = backward_views<FMT, false, false, kMaxDiffViews>(p + v, m, ckpt + (size_t)v * stride, stride, per_ray,
                                                                  dl + (size_t)v * npix, gt, s);

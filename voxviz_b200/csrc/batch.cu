@@ -177,7 +177,7 @@ static int batch_launch(vv_ctx* c, const vv_batch_view* views, int32_t n, const 
             std::memset(&v, 0, sizeof(v));
             v.p.u = *u;
             set_divisors(v.p);
-            set_nodes(v.p, t.nodes, t.dim);
+            set_nodes(v.p, t.pool());
             for (int a = 0; a < 3; ++a) v.p.slots[a] = bv.ctx->slots[a];
             v.p.bricks = bv.ctx->bricks;
             v.p.cell_mask = ctx_cell_mask(bv.ctx);

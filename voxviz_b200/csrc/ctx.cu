@@ -185,8 +185,10 @@ int vv_ctx_destroy(vv_ctx* c) {
     if (!c) return VV_OK;
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
-    for (auto& t : c->trees)
+    for (auto& t : c->trees) {
         if (t.nodes) cudaFree(t.nodes);
+        if (t.walk) cudaFree(t.walk);
+    }
     if (c->bricks && !c->bricks_external) cudaFree(c->bricks);
     void* bufs[] = {c->d_status, c->d_jitter, c->d_usage, c->d_mask, c->d_counts, c->d_offsets,
                     c->d_up_slots, c->d_up_bricks, c->d_patches, c->d_grid_words, c->d_batch, c->grads,
@@ -227,6 +229,13 @@ int vv_ctx_device_status(vv_ctx* c, int32_t* status, int32_t clear) {
     return VV_OK;
 }
 
+// The words of a node pool travel in slabs of 16 MB (one z slice at least): the
+// staging is what bounds the pool beside its words and walk records.
+static size_t slice_bytes(const DeviceTree& t) { return (size_t)t.dim[0] * t.dim[1] * sizeof(uint2); }
+static int node_slab(const DeviceTree& t) {
+    return std::min(t.dim[2], (int)std::max<size_t>(1, ((size_t)16 << 20) / slice_bytes(t)));
+}
+
 int vv_nodepool_upload(vv_ctx* c, int32_t tree, const uint32_t* words, int32_t dx, int32_t dy, int32_t dz) {
     if (!c || !words || tree < 0 || tree >= VV_MAX_TREES) return fail(c, VV_ERR_ARG, "bad node pool arguments");
     if (dx <= 0 || dy <= 0 || dz <= 0 || (dx & 1) || (dy & 1) || (dz & 1) || dx > 1024 || dy > 1024 || dz > 1024)
@@ -236,24 +245,33 @@ int vv_nodepool_upload(vv_ctx* c, int32_t tree, const uint32_t* words, int32_t d
     const size_t cells = (size_t)dx * dy * dz;
     if (t.nodes && t.cells != cells) {
         cudaFree(t.nodes);
-        t.nodes = nullptr;
+        if (t.walk) cudaFree(t.walk);
+        t.nodes = t.walk = nullptr;
     }
-    if (!t.nodes) {
-        // the words and, behind them, the walk's records (walknode.h)
-        cudaError_t e = cudaMalloc(&t.nodes, 2 * cells * sizeof(uint2));
-        if (e != cudaSuccess) {
-            t.nodes = nullptr;
-            return fail(c, VV_ERR_OOM, "cudaMalloc node pool");
-        }
+    const bool fresh = !t.nodes;
+    if (fresh && cudaMalloc(&t.nodes, cells * sizeof(uint2)) != cudaSuccess) {
+        t.nodes = nullptr;
+        return fail(c, VV_ERR_OOM, "cudaMalloc node pool");
     }
     t.cells = cells;
     t.dim[0] = dx;
     t.dim[1] = dy;
     t.dim[2] = dz;
-    int rc = ensure(c, (void**)&c->d_grid_words, &c->grid_words_cap, cells * sizeof(uint2), "node staging");
+    const int slab = node_slab(t);
+    int rc = ensure(c, (void**)&c->d_grid_words, &c->grid_words_cap, slab * slice_bytes(t), "node staging");
     if (rc) return rc;
-    VV_CUDA(c, cudaMemcpyAsync(c->d_grid_words, words, cells * sizeof(uint2), cudaMemcpyHostToDevice, c->stream));
-    VV_CUDA(c, launch_node_upload(c->d_grid_words, t.nodes, t.dim, c->stream));
+    // the walk's records only with the words (a captured draw keeps what there
+    // is), and after all else that the upload needs
+    if (fresh && cudaMalloc(&t.walk, cells * sizeof(uint2)) != cudaSuccess) {
+        t.walk = nullptr;
+        cudaGetLastError();
+    }
+    for (int z = 0; z < dz; z += slab) {
+        const int nz = std::min(slab, dz - z);
+        VV_CUDA(c, cudaMemcpyAsync(c->d_grid_words, (const char*)words + z * slice_bytes(t), nz * slice_bytes(t),
+                                   cudaMemcpyHostToDevice, c->stream));
+        VV_CUDA(c, launch_node_upload(c->d_grid_words, t.pool(), z, nz, c->stream));
+    }
     VV_CUDA(c, cudaStreamSynchronize(c->stream));
     return VV_OK;
 }
@@ -273,7 +291,7 @@ int vv_nodepool_patch(vv_ctx* c, int32_t tree, const vv_node_patch* patches, int
     VV_CUDA(c, cudaStreamSynchronize(c->stream));  // staging buffer reuse
     std::memcpy(c->h_stage, patches, bytes);
     VV_CUDA(c, cudaMemcpyAsync(c->d_patches, c->h_stage, bytes, cudaMemcpyHostToDevice, c->stream));
-    VV_CUDA(c, launch_node_patch(c->d_patches, n, t.nodes, t.dim, c->d_status, c->stream));
+    VV_CUDA(c, launch_node_patch(c->d_patches, n, t.pool(), c->d_status, c->stream));
     return VV_OK;
 }
 
@@ -282,10 +300,15 @@ int vv_nodepool_download(vv_ctx* c, int32_t tree, uint32_t* words) {
     DeviceTree& t = c->trees[tree];
     if (!t.nodes) return fail(c, VV_ERR_STATE, "node pool not uploaded");
     cudaSetDevice(c->device);
-    int rc = ensure(c, (void**)&c->d_grid_words, &c->grid_words_cap, t.cells * sizeof(uint2), "node staging");
+    const int slab = node_slab(t);
+    int rc = ensure(c, (void**)&c->d_grid_words, &c->grid_words_cap, slab * slice_bytes(t), "node staging");
     if (rc) return rc;
-    VV_CUDA(c, launch_node_download(t.nodes, c->d_grid_words, t.dim, c->stream));
-    VV_CUDA(c, cudaMemcpyAsync(words, c->d_grid_words, t.cells * sizeof(uint2), cudaMemcpyDeviceToHost, c->stream));
+    for (int z = 0; z < t.dim[2]; z += slab) {
+        const int nz = std::min(slab, t.dim[2] - z);
+        VV_CUDA(c, launch_node_download(t.pool(), c->d_grid_words, z, nz, c->stream));
+        VV_CUDA(c, cudaMemcpyAsync((char*)words + z * slice_bytes(t), c->d_grid_words, nz * slice_bytes(t),
+                                   cudaMemcpyDeviceToHost, c->stream));
+    }
     VV_CUDA(c, cudaStreamSynchronize(c->stream));
     return VV_OK;
 }
@@ -483,7 +506,7 @@ static int diff_params(vv_ctx* c, int32_t tree, const vv_uniforms* u, RaycastPar
     std::memset(&p, 0, sizeof(p));
     p.u = *u;
     set_divisors(p);
-    set_nodes(p, t.nodes, t.dim);
+    set_nodes(p, t.pool());
     for (int a = 0; a < 3; ++a) p.slots[a] = c->slots[a];
     p.bricks = c->bricks;
     p.cell_mask = ctx_cell_mask(c);
@@ -667,7 +690,7 @@ int vv_render(vv_ctx* c, int32_t tree, const vv_uniforms* u, const vv_frame_out*
         std::memset(&p, 0, sizeof(p));
         p.u = *u;
         set_divisors(p);
-        set_nodes(p, t.nodes, t.dim);
+        set_nodes(p, t.pool());
         p.bricks = c->bricks;
         p.cell_mask = ctx_cell_mask(c);
         p.slots[0] = c->slots[0];
@@ -684,8 +707,8 @@ int vv_render(vv_ctx* c, int32_t tree, const vv_uniforms* u, const vv_frame_out*
             p.grads = c->grads;
             p.grad_fmt = c->grad_fmt;
         }
-        // the refill form walks the unit box only
-        if (c->raycast_mode == VV_RAYCAST_REFILL && !u->compute_lighting && is_unit_box(*u)) {
+        // the refill form has the unit box's walk only
+        if (c->raycast_mode == VV_RAYCAST_REFILL && !u->compute_lighting && takes_unit_walk(p)) {
             if (!c->d_refill_counter) VV_CUDA(c, cudaMalloc(&c->d_refill_counter, sizeof(unsigned int)));
             VV_CUDA(c, launch_raycast_refill(c->fmt, p, c->d_refill_counter, c->stream));
         } else if (c->raycast_mode == VV_RAYCAST_STAGED && !u->compute_lighting && c->fmt == VV_FMT_RGBA8) {
@@ -814,7 +837,7 @@ int vv_measure_footprint_views(vv_ctx* c, int32_t tree, const vv_uniforms* us, i
         std::memset(&p, 0, sizeof(p));
         p.u = us[i];
         set_divisors(p);
-        set_nodes(p, t.nodes, t.dim);
+        set_nodes(p, t.pool());
         for (int a = 0; a < 3; ++a) p.slots[a] = c->slots[a];
         p.bricks = c->bricks;
         p.jitter = c->d_jitter;

@@ -7,13 +7,16 @@
 #include <string>
 
 #include "../../include/voxviz_b200.h"
+#include "nodepool.h"
 
 namespace vv {
 
 struct DeviceTree {
-    uint2* nodes = nullptr;  // block-linear node pool, then its walk records (walknode.h)
+    uint2* nodes = nullptr;  // block-linear node pool
+    uint2* walk = nullptr;   // its walk records (walknode.h), or nullptr
     int dim[3] = {0, 0, 0};
     size_t cells = 0;
+    NodePool pool() const { return NodePool{nodes, walk, {dim[0], dim[1], dim[2]}}; }
 };
 
 int vv_max_iterations(const vv_uniforms* u);

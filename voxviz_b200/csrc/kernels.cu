@@ -308,84 +308,81 @@ __device__ __forceinline__ size_t block_linear(uint32_t x, uint32_t y, uint32_t 
     return blk * 8u + ((x & 1u) | ((y & 1u) << 1) | ((z & 1u) << 2));
 }
 
-// Node i's words and its walk record.
-__device__ __forceinline__ void write_node(uint2* __restrict__ nodes, size_t i, uint2 w, int dx, int dy, int dz) {
-    nodes[i] = w;
-    nodes[(size_t)dx * dy * dz + i] = make_uint2(walk_link(w.x, dx, dy, dz), w.y);
+// Node i's words and, of a pool that has them, its walk record.
+__device__ __forceinline__ void write_node(const NodePool& n, size_t i, uint2 w) {
+    n.words[i] = w;
+    if (n.walk) n.walk[i] = make_uint2(walk_link(w.x, n.dim[0], n.dim[1], n.dim[2]), w.y);
 }
 
-__global__ void node_upload_kernel(const uint2* __restrict__ grid, uint2* __restrict__ nodes, int dx, int dy,
-                                   int dz) {
-    const size_t total = (size_t)dx * dy * dz;
+// Slices [z0, z0 + nz) of the grid, `grid` their words in texture order.
+__global__ void node_upload_kernel(const uint2* __restrict__ grid, const NodePool n, int z0, int nz) {
+    const int dx = n.dim[0], dy = n.dim[1];
+    const size_t total = (size_t)dx * dy * nz;
     for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < total; g += (size_t)gridDim.x * blockDim.x) {
-        uint32_t x = (uint32_t)(g % dx), y = (uint32_t)((g / dx) % dy), z = (uint32_t)(g / ((size_t)dx * dy));
-        write_node(nodes, block_linear(x, y, z, dx, dy), grid[g], dx, dy, dz);
+        uint32_t x = (uint32_t)(g % dx), y = (uint32_t)((g / dx) % dy), z = z0 + (uint32_t)(g / ((size_t)dx * dy));
+        write_node(n, block_linear(x, y, z, dx, dy), grid[g]);
     }
 }
 
-__global__ void node_download_kernel(const uint2* __restrict__ nodes, uint2* __restrict__ grid, int dx, int dy,
-                                     int dz) {
-    const size_t total = (size_t)dx * dy * dz;
+__global__ void node_download_kernel(const NodePool n, uint2* __restrict__ grid, int z0, int nz) {
+    const int dx = n.dim[0], dy = n.dim[1];
+    const size_t total = (size_t)dx * dy * nz;
     for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < total; g += (size_t)gridDim.x * blockDim.x) {
-        uint32_t x = (uint32_t)(g % dx), y = (uint32_t)((g / dx) % dy), z = (uint32_t)(g / ((size_t)dx * dy));
-        grid[g] = nodes[block_linear(x, y, z, dx, dy)];
+        uint32_t x = (uint32_t)(g % dx), y = (uint32_t)((g / dx) % dy), z = z0 + (uint32_t)(g / ((size_t)dx * dy));
+        grid[g] = n.words[block_linear(x, y, z, dx, dy)];
     }
 }
 
-__global__ void node_patch_kernel(const vv_node_patch* __restrict__ patches, int n, uint2* __restrict__ nodes,
-                                  int dx, int dy, int dz, int* status) {
+__global__ void node_patch_kernel(const vv_node_patch* __restrict__ patches, int count, const NodePool n, int* status) {
     // The host hands over at most one patch per node (the last one it made),
     // so the parallel writes are order-independent.
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= count) return;
     const vv_node_patch q = patches[i];
-    if (q.x >= (uint32_t)dx || q.y >= (uint32_t)dy || q.z >= (uint32_t)dz) {
+    if (q.x >= (uint32_t)n.dim[0] || q.y >= (uint32_t)n.dim[1] || q.z >= (uint32_t)n.dim[2]) {
         set_status(status, VV_ERR_BOUNDS);
         return;
     }
-    write_node(nodes, block_linear(q.x, q.y, q.z, dx, dy), make_uint2(q.word0, q.word1), dx, dy, dz);
+    write_node(n, block_linear(q.x, q.y, q.z, n.dim[0], n.dim[1]), make_uint2(q.word0, q.word1));
 }
 
 __global__ void node_patch_staged_kernel(const vv_node_patch* patches, const volatile uint32_t* count,
-                                         uint32_t max_patches, uint2* __restrict__ nodes, int dx, int dy, int dz,
-                                         int* status) {
+                                         uint32_t max_patches, const NodePool n, int* status) {
     __shared__ uint32_t s_n;  // one read of the count per CTA
     if (threadIdx.x == 0) s_n = min(*count, max_patches);
     __syncthreads();
-    const uint32_t n = s_n;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t total = s_n;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const vv_node_patch q = patches[i];
-        if (q.x >= (uint32_t)dx || q.y >= (uint32_t)dy || q.z >= (uint32_t)dz) {
+        if (q.x >= (uint32_t)n.dim[0] || q.y >= (uint32_t)n.dim[1] || q.z >= (uint32_t)n.dim[2]) {
             set_status(status, VV_ERR_BOUNDS);
             continue;
         }
-        write_node(nodes, block_linear(q.x, q.y, q.z, dx, dy), make_uint2(q.word0, q.word1), dx, dy, dz);
+        write_node(n, block_linear(q.x, q.y, q.z, n.dim[0], n.dim[1]), make_uint2(q.word0, q.word1));
     }
 }
 
 cudaError_t launch_node_patch_staged(const vv_node_patch* patches, const uint32_t* count, uint32_t max_patches,
-                                     uint2* nodes, const int dim[3], int* status, cudaStream_t s) {
+                                     const NodePool& pool, int* status, cudaStream_t s) {
     if (max_patches == 0) return cudaSuccess;
     const unsigned grid = (unsigned)std::min<uint32_t>((max_patches + 255) / 256, 1184u);
-    node_patch_staged_kernel<<<grid, 256, 0, s>>>(patches, count, max_patches, nodes, dim[0], dim[1], dim[2],
-                                                  status);
+    node_patch_staged_kernel<<<grid, 256, 0, s>>>(patches, count, max_patches, pool, status);
     return cudaGetLastError();
 }
 
-cudaError_t launch_node_upload(const uint32_t* grid_words, uint2* nodes, const int dim[3], cudaStream_t s) {
-    node_upload_kernel<<<592, 256, 0, s>>>((const uint2*)grid_words, nodes, dim[0], dim[1], dim[2]);
+cudaError_t launch_node_upload(const uint32_t* grid_words, const NodePool& pool, int z0, int nz, cudaStream_t s) {
+    node_upload_kernel<<<592, 256, 0, s>>>((const uint2*)grid_words, pool, z0, nz);
     return cudaGetLastError();
 }
 
-cudaError_t launch_node_download(const uint2* nodes, uint32_t* grid_words, const int dim[3], cudaStream_t s) {
-    node_download_kernel<<<592, 256, 0, s>>>(nodes, (uint2*)grid_words, dim[0], dim[1], dim[2]);
+cudaError_t launch_node_download(const NodePool& pool, uint32_t* grid_words, int z0, int nz, cudaStream_t s) {
+    node_download_kernel<<<592, 256, 0, s>>>(pool, (uint2*)grid_words, z0, nz);
     return cudaGetLastError();
 }
 
-cudaError_t launch_node_patch(const vv_node_patch* patches, int n, uint2* nodes, const int dim[3], int* status,
-                              cudaStream_t s) {
+cudaError_t launch_node_patch(const vv_node_patch* patches, int n, const NodePool& pool, int* status, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    node_patch_kernel<<<(n + 255) / 256, 256, 0, s>>>(patches, n, nodes, dim[0], dim[1], dim[2], status);
+    node_patch_kernel<<<(n + 255) / 256, 256, 0, s>>>(patches, n, pool, status);
     return cudaGetLastError();
 }
 

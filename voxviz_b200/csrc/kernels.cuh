@@ -8,6 +8,7 @@
 
 #include "../../include/voxviz_b200.h"
 #include "lod_bound.h"
+#include "nodepool.h"
 #include "walknode.h"
 
 namespace vv {
@@ -16,7 +17,7 @@ namespace vv {
 struct RaycastParams {
     vv_uniforms u;
     const uint2* nodes;      // node pool, block-linear: 8 nodes of a 2x2x2 cell contiguous
-    const uint2* walk;       // the same nodes as the walk reads them (walknode.h)
+    const uint2* walk;       // the same nodes as the walk reads them (walknode.h), or nullptr
     BlockDiv row, slice;     // node blocks per row and per slice of the grid
     int node_dim[3];         // node-pool grid dims (even)
     const void* bricks;      // brick pool, slot-major brick-linear texels
@@ -40,13 +41,13 @@ struct RaycastParams {
     int color8;              // colour as RGBA8 unorm: color is read as uint32_t[H*W]
 };
 
-// The node pool of a launch (host): its walk records follow its words.
-inline void set_nodes(RaycastParams& p, const uint2* nodes, const int dim[3]) {
-    p.nodes = nodes;
-    p.walk = nodes + (size_t)dim[0] * dim[1] * dim[2];
-    for (int a = 0; a < 3; ++a) p.node_dim[a] = dim[a];
-    p.row = make_block_div((uint32_t)dim[0] / 2u);
-    p.slice = make_block_div((uint32_t)dim[0] / 2u * ((uint32_t)dim[1] / 2u));
+// The node pool of a launch (host).
+inline void set_nodes(RaycastParams& p, const NodePool& n) {
+    p.nodes = n.words;
+    p.walk = n.walk;
+    for (int a = 0; a < 3; ++a) p.node_dim[a] = n.dim[a];
+    p.row = make_block_div((uint32_t)n.dim[0] / 2u);
+    p.slice = make_block_div((uint32_t)n.dim[0] / 2u * ((uint32_t)n.dim[1] / 2u));
 }
 
 // Whether the volume box is [0,1]^3.
@@ -55,6 +56,9 @@ inline bool is_unit_box(const vv_uniforms& u) {
         if (u.vol_extent_min[a] != 0.0f || u.vol_extent_max[a] != 1.0f) return false;
     return true;
 }
+
+// Whether a launch takes the unit box's walk (host; unit_walk on the device).
+inline bool takes_unit_walk(const RaycastParams& p) { return p.walk && is_unit_box(p.u); }
 
 // What RaycastParams holds derived from its uniforms (host).
 inline void set_divisors(RaycastParams& p) {
@@ -126,17 +130,15 @@ cudaError_t launch_compact(const CompactParams& p, cudaStream_t s);
 // loff[l], dims lw[l] x lh[l]).
 cudaError_t launch_pyramid_levels(uint32_t* counts, uint32_t* offsets, const int* lw, const int* lh,
                                   const long long* loff, int first, int levels, cudaStream_t s);
-cudaError_t launch_node_upload(const uint32_t* grid_words, uint2* nodes, const int dim[3],
-                               cudaStream_t s);
-cudaError_t launch_node_download(const uint2* nodes, uint32_t* grid_words, const int dim[3],
-                                 cudaStream_t s);
+// Slices [z0, z0 + nz) of the pool's grid from or to their words in texture order.
+cudaError_t launch_node_upload(const uint32_t* grid_words, const NodePool& pool, int z0, int nz, cudaStream_t s);
+cudaError_t launch_node_download(const NodePool& pool, uint32_t* grid_words, int z0, int nz, cudaStream_t s);
 // Patches and their count read on the device (at most max_patches): a
 // count-independent launch for CUDA graphs.  Device copies of both make it
 // fast (mapped host memory costs a bus round trip per CTA).
 cudaError_t launch_node_patch_staged(const vv_node_patch* patches, const uint32_t* count, uint32_t max_patches,
-                                     uint2* nodes, const int dim[3], int* status, cudaStream_t s);
-cudaError_t launch_node_patch(const vv_node_patch* patches, int n, uint2* nodes, const int dim[3],
-                              int* status, cudaStream_t s);
+                                     const NodePool& pool, int* status, cudaStream_t s);
+cudaError_t launch_node_patch(const vv_node_patch* patches, int n, const NodePool& pool, int* status, cudaStream_t s);
 cudaError_t launch_brick_scatter(const uint32_t* slots, int n, const void* src, void* pool,
                                  size_t brick_bytes, long long total_slots, int* status,
                                  cudaStream_t s);

@@ -520,9 +520,11 @@ struct RayState {
 
 enum { kSampleConst = 0, kSampleBrick = 1 };
 
-// Whether the volume box is [0,1]^3.
-__device__ __forceinline__ bool unit_box(const vv_uniforms& u) {
-    return u.vol_extent_min[0] == 0.0f && u.vol_extent_min[1] == 0.0f && u.vol_extent_min[2] == 0.0f &&
+// Whether a draw takes the unit box's walk: its volume box is [0,1]^3 and the
+// pool has walk records.
+__device__ __forceinline__ bool unit_walk(const RaycastParams& p) {
+    const vv_uniforms& u = p.u;
+    return p.walk && u.vol_extent_min[0] == 0.0f && u.vol_extent_min[1] == 0.0f && u.vol_extent_min[2] == 0.0f &&
            u.vol_extent_max[0] == 1.0f && u.vol_extent_max[1] == 1.0f && u.vol_extent_max[2] == 1.0f;
 }
 
@@ -1321,7 +1323,7 @@ __device__ __forceinline__ void walk_warp(const RaycastParams& p, const WalkCons
 
 // walk() runs a ray's segments until its walk has ended; all 32 lanes of a warp
 // call it, `alive` the ones that have a ray.  UNIT: the volume box is [0,1]^3
-// (unit_box), as compute_uniforms makes it; each pixel body keeps the other
+// (unit_walk), as compute_uniforms makes it; each pixel body keeps the other
 // boxes in a function of its own, out of line, so that they cost the unit box
 // neither registers nor instruction cache.
 template <int FMT, bool COUNT, class V, bool UNIT, int AHEAD, bool LIT = false, bool STAGED = false>
@@ -1421,7 +1423,7 @@ __device__ __noinline__ void pixel_body_box(const RaycastParams& p, int px, int 
 template <int FMT, bool COUNT, int AHEAD, bool LIT = false, bool STAGED = false>
 __device__ __forceinline__ void render_pixel(const RaycastParams& p, int px, int py, const PathSlots& path) {
     if (COUNT) pixel_body<FMT, true, false, 1, LIT, false>(p, px, py, path);
-    else if (unit_box(p.u)) pixel_body<FMT, false, true, AHEAD, LIT, STAGED>(p, px, py, path);
+    else if (unit_walk(p)) pixel_body<FMT, false, true, AHEAD, LIT, STAGED>(p, px, py, path);
     else pixel_body_box<FMT, LIT>(p, px, py);
 }
 

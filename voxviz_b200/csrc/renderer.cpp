@@ -658,7 +658,7 @@ int GigaVoxelsRenderer::flush_device() {
                                       (long long)total_slots_, ctx_->d_status, ctx_->stream)
                  : launch_produce_bricks(dterrain_->view(), d_fjobs_, (int)n, pool, d_.fmt, ctx_cell_mask_rw(ctx_),
                                          (long long)total_slots_, ctx_->d_status, ctx_->stream)) != cudaSuccess ||
-        launch_node_patch(d_fpatch_, (int)np, t.nodes, t.dim, ctx_->d_status, ctx_->stream) != cudaSuccess)
+        launch_node_patch(d_fpatch_, (int)np, t.pool(), ctx_->d_status, ctx_->stream) != cudaSuccess)
         return VV_ERR_CUDA;
     touched_.clear();
     pending_nodes_.clear();
@@ -1006,7 +1006,7 @@ int GigaVoxelsRenderer::enqueue_uploads() {
                                         ctx_cell_mask_rw(ctx_), (long long)total_slots_, ctx_->d_status, ctx_->stream);
     if (pe != cudaSuccess) return VV_ERR_CUDA;
     const DeviceTree& t = ctx_->trees[0];
-    if (launch_node_patch_staged(d_def_patches_, d_def_counts_ + 1, def_patch_cap_, t.nodes, t.dim, ctx_->d_status,
+    if (launch_node_patch_staged(d_def_patches_, d_def_counts_ + 1, def_patch_cap_, t.pool(), ctx_->d_status,
                                  ctx_->stream) != cudaSuccess)
         return VV_ERR_CUDA;
     // the staging's generation, recorded as applied after its patches

@@ -3,7 +3,7 @@
 // A node's reference word (GpuDataStruct word 0) points at its children by the
 // grid position of their 2x2x2 block; following it costs the walk an unpack, a
 // bounds check and the block-linear index per level.  The pool therefore also
-// keeps, right behind its words, one 8-byte record per node with that index
+// keeps (memory allowing, nodepool.h) one 8-byte record per node with that index
 // worked out when the word is written:
 //   x: the resident and constant bits of word 0, and in the low 27 bits the
 //      child block (its 8 nodes are 8*block .. 8*block+7), 0 for no children,
