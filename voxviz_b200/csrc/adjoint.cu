@@ -28,7 +28,7 @@ using namespace rc;
 namespace {
 
 // The views of a launch: views of one size over the same pools.
-constexpr int kMaxDiffViews = 16;  // 472 bytes each of the launch parameters
+constexpr int kMaxDiffViews = 16;  // 480 bytes each of the launch parameters
 template <int VIEWS>
 struct DiffViews {
     RaycastParams p[VIEWS];

@@ -4,7 +4,7 @@
 // all views' pixel tiles from a device work queue (one atomic counter; tiles
 // numbered view by view, row-major inside a view).  The views' RaycastParams (uniforms +
 // the pools of each view's octree) travel by value in the kernel's parameter
-// space, up to kMaxLaunchViews views per launch (64 with the 480-byte view
+// space, up to kMaxLaunchViews views per launch (64 with the 488-byte view
 // record; larger batches launch in chunks), so a
 // CTA reads its view's parameters from the constant bank as the single-view
 // ray cast does, and runs render_pixel, the vv_render ray cast, on every
@@ -35,7 +35,7 @@ struct BatchView {
 };
 
 // The views of one launch.  Kernel parameters may take 32,764 bytes.
-constexpr int kMaxLaunchViews = 64;  // 480 bytes each
+constexpr int kMaxLaunchViews = 64;  // 488 bytes each
 struct BatchParams {
     int n;            // views
     int total_tiles;  // tiles of all n views

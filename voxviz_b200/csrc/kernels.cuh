@@ -38,6 +38,7 @@ struct RaycastParams {
     float rstep;
     lodb::Consts lodk;       // set_divisors: constants of the LOD certificate (lod_bound.h)
     float bstep_texel[3];    // set_divisors: texels a brick sample moves along a unit direction
+    int pass_steps;          // set_divisors: samples a brick may take to be passed over by projections
     int color8;              // colour as RGBA8 unorm: color is read as uint32_t[H*W]
 };
 
@@ -70,7 +71,12 @@ inline void set_divisors(RaycastParams& p) {
     const auto v3 = [](const float* f) { return lodb::V3{f[0], f[1], f[2]}; };
     p.lodk = lodb::make_consts(v3(u.camera_position), v3(u.camera_up), v3(u.camera_left), u.root_voxel_half_size,
                                u.lod_scalar, u.pixel_size, u.oct_tree_depth_minus_one, is_unit_box(u));
-    for (int a = 0; a < 3; ++a) p.bstep_texel[a] = u.brick_step_vector[a] * u.brick_pool_dimension[a];
+    // (a step that is not finite has no first and last sample to bound the others by)
+    p.pass_steps = 128;
+    for (int a = 0; a < 3; ++a) {
+        p.bstep_texel[a] = u.brick_step_vector[a] * u.brick_pool_dimension[a];
+        if (!std::isfinite(p.bstep_texel[a])) p.pass_steps = 0;
+    }
 }
 
 // Pyramid/compaction launch state.

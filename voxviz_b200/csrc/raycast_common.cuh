@@ -816,6 +816,8 @@ __device__ __forceinline__ uint32_t slot_of(const RaycastParams& p, uint32_t bw)
 // the last sample bound those between, per axis; they are off from the
 // shader's sums by less than 0.01 texel for up to 128 samples (a sum of
 // coordinates below 1 in pools of at most 1020 texels rounds by 6e-5 texel).
+// A count out of 1..pass_steps (set_divisors; a quotient by a tiny step
+// overflows) shows nothing.
 __device__ __forceinline__ bool brick_empty(const RaycastParams& p, const WalkConsts& k, F3 brp, F3 dir, int n,
                                             uint32_t slot) {
     const uint32_t occ = __ldg(p.cell_mask + (size_t)slot * kCellMaskWords + kOccupancyWord);
@@ -823,7 +825,7 @@ __device__ __forceinline__ bool brick_empty(const RaycastParams& p, const WalkCo
     const F3 u0 = f3(fmaf(brp.x, k.bdim.x, 0.5f), fmaf(brp.y, k.bdim.y, 0.5f), fmaf(brp.z, k.bdim.z, 0.5f));
     const F3 u1 = f3(fmaf(m * dir.x, p.bstep_texel[0], u0.x), fmaf(m * dir.y, p.bstep_texel[1], u0.y),
                      fmaf(m * dir.z, p.bstep_texel[2], u0.z));
-    bool in = n <= 128, empty = false;
+    bool in = (unsigned)(n - 1) < (unsigned)p.pass_steps, empty = false;
     const float a0[3] = {u0.x, u0.y, u0.z}, a1[3] = {u1.x, u1.y, u1.z};
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
