@@ -98,7 +98,7 @@ struct Consts {
     int max_level;
     bool ok;
     // deep_levels: the deepest level's half voxel size squared and times theta,
-    // the smallest |a|^2 it covers (a huge one: none)
+    // the smallest |a|^2 it covers (NaN: none; a far camera's |a|^2 may be infinite)
     float quick_vh2, quick_theta, quick_min;
 };
 
@@ -150,7 +150,7 @@ VV_HD Consts make_consts(V3 C, V3 up, V3 left, float rvh, float lod, float pixel
     }
     const float dm = k.d0 / (amin > 1e-6f ? amin : 1e-6f) + k.d1;
     k.quick_min = k.ok && max_level >= kDeepTries && max_level < 60 && amin > 1e-6f && k.need >= 12.6f * dm * dm
-                      ? amin * amin * 1.001f : 3e38f;
+                      ? amin * amin * 1.001f : NAN;
     return k;
 }
 
