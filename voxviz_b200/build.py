@@ -29,7 +29,7 @@ CU_SOURCES = ["kernels.cu", "ctx.cu", "noalloc.cu", "production.cu", "adjoint.cu
               "compact.cu"]
 CPP_SOURCES = ["terrain.cpp", "octree.cpp", "gradients.cpp", "gvfile.cpp", "renderer.cpp", "scene.cpp", "capi.cpp"]
 HEADERS = ["kernels.cuh", "cellmask.cuh", "select.cuh", "compact.h", "dxt.h", "ctx.h", "terrain.h", "octree.h", "gvfile.h", "scene.h", "handles.h", "renderer.h", "production.h", "raycast_common.cuh",
-           "lod_bound.h", "walknode.h", "nodepool.h", "gradients.h", "fixed_div.h"]
+           "lod_bound.h", "walknode.h", "nodepool.h", "ckpt_layout.h", "gradients.h", "fixed_div.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

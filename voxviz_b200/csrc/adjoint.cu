@@ -19,6 +19,7 @@
 // cross more segments than there are records.  The control flow (descent, step counts, early
 // termination) is that of the forward and is held fixed, as any reverse-mode
 // derivative of this shader does.
+#include "ckpt_layout.h"
 #include "raycast_common.cuh"
 
 namespace vv {
@@ -44,7 +45,7 @@ struct Ckpt {
     float2 p0, p1;
     uint2 w;
 };
-constexpr int kRecordsPerSlot = 2;  // a caller's record slot has 48 bytes
+static_assert(sizeof(Ckpt) == kRecordBytes && alignof(Ckpt) == 8, "records are 24 bytes of 8-byte vectors");
 enum { kRecBrick = 0, kRecConst = 1, kRecWalk = 2 };
 
 struct CkptVisitor {
@@ -57,7 +58,7 @@ struct CkptVisitor {
     int* status;
     __device__ __forceinline__ void start(Ckpt* out_, int per_ray, int* status_) {
         out = out_;
-        cap = per_ray * kRecordsPerSlot;
+        cap = record_cap(per_ray);
         count = 0;
         last = -kCkptEvery;
         segments = cap - max(1, cap / 4);
@@ -334,7 +335,7 @@ __device__ __forceinline__ void forward_pixel(const RaycastParams& p, int px, in
     bool ok = true;
     const WalkConsts k = walk_consts(p, UNIT ? __ldg(p.walk) : fetch_node<false>(p, 0, 0, 0, ok));
     CkptVisitor vis;
-    vis.start(ckpt + pix * (size_t)(per_ray * kRecordsPerSlot), per_ray, p.status);
+    vis.start(ckpt + pix * ray_records(per_ray), per_ray, p.status);
     RayState s;
     s.dst = make_float4(0.f, 0.f, 0.f, 0.f);
     s.nsamples = 0;
@@ -422,7 +423,7 @@ __device__ __forceinline__ void backward_pixel(const RaycastParams& p, int px, i
     bool more = C != 0 && total != 0 && (g.x != 0.f || g.y != 0.f || g.z != 0.f || g.w != 0.f) &&
                 ray_origin(u, k, px, py, pos);
     ray_start(p, k, inside ? px : 0, inside ? py : 0, pos, s0);  // direction of this ray
-    const Ckpt* ck = ckpt + pix * (size_t)(per_ray * kRecordsPerSlot);
+    const Ckpt* ck = ckpt + pix * ray_records(per_ray);
     uint32_t c_slot = 0xFFFFFFFFu;  // the last slot scattered into and its gradient row
     int c_row = -1;
     Piece piece;
@@ -533,7 +534,7 @@ __device__ __forceinline__ void backward_pixel_box(const RaycastParams& p, int p
     F3 pos;
     if (!ray_origin(u, k, px, py, pos)) return;
     ray_start(p, k, px, py, pos, s0);
-    const Ckpt* ck = ckpt + pix * (size_t)(per_ray * kRecordsPerSlot);
+    const Ckpt* ck = ckpt + pix * ray_records(per_ray);
     uint32_t c_slot = 0xFFFFFFFFu;
     int c_row = -1;
     Piece piece;
@@ -650,15 +651,7 @@ cudaError_t launch_spread_reduce(const GradTarget& grad, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-namespace {
-// The headers' bytes, rounded up to the records' alignment (an odd number of
-// pixels would leave the 16-byte record vectors on an 8-byte boundary).
-size_t hdr_bytes(int w, int h) { return ((size_t)w * h * sizeof(int2) + 15) / 16 * 16; }
-}  // namespace
-
-size_t ckpt_bytes(int w, int h, int per_ray) {
-    return hdr_bytes(w, h) + (size_t)w * h * (size_t)per_ray * kRecordsPerSlot * sizeof(Ckpt);
-}
+size_t ckpt_bytes(int w, int h, int per_ray) { return ckpt_buffer_bytes(w, h, per_ray); }
 
 namespace {
 
@@ -669,7 +662,7 @@ cudaError_t forward_views(const RaycastParams* p, int n, char* ckpt, size_t stri
     const int W = p->u.width, H = p->u.height;
     DiffViews<VIEWS> dv;
     for (int v = 0; v < n; ++v) dv.p[v] = p[v];
-    const size_t hdr = hdr_bytes(W, H);
+    const size_t hdr = ckpt_header_bytes(W, H);
     const int rays = rays_per_warp((long long)n * W * H);
     const dim3 grid = warp_grid(rays, W, H, n);
     if (rays == 4) forward_ckpt_kernel<FMT, VIEWS, 4><<<grid, 128, 0, s>>>(dv, ckpt, stride, hdr, per_ray);
@@ -684,7 +677,7 @@ cudaError_t backward_views(const RaycastParams* p, int n, const char* ckpt, size
     const int W = p->u.width, H = p->u.height;
     DiffViews<VIEWS> dv;
     for (int v = 0; v < n; ++v) dv.p[v] = p[v];
-    const size_t hdr = hdr_bytes(W, H);
+    const size_t hdr = ckpt_header_bytes(W, H);
     // (the forms for checks and comparisons take full warps)
     const int rays = F64 || WSUM ? 32 : rays_per_warp((long long)n * W * H);
     const dim3 grid = warp_grid(rays, W, H, n);
@@ -707,7 +700,7 @@ cudaError_t backward_view(const RaycastParams* p, const char* ckpt, size_t strid
                           const GradTarget& gt, cudaStream_t s) {
     if (takes_unit_walk(*p)) return backward_views<FMT, F64, WSUM, 1>(p, 1, ckpt, stride, per_ray, dl, gt, s);
     const int W = p->u.width, H = p->u.height;
-    backward_box_kernel<FMT, F64, WSUM><<<warp_grid(32, W, H), 128, 0, s>>>(*p, ckpt, hdr_bytes(W, H), per_ray, dl, gt);
+    backward_box_kernel<FMT, F64, WSUM><<<warp_grid(32, W, H), 128, 0, s>>>(*p, ckpt, ckpt_header_bytes(W, H), per_ray, dl, gt);
     return cudaGetLastError();
 }
 
