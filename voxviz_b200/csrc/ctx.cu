@@ -518,7 +518,7 @@ static int diff_params(vv_ctx* c, int32_t tree, const vv_uniforms* u, RaycastPar
 
 // The launch parameters of a call's views, which have one size.
 static int diff_views(vv_ctx* c, int32_t tree, const vv_uniforms* us, int32_t n, std::vector<RaycastParams>& p) {
-    if (!us || n <= 0 || n > 65536) return fail(c, VV_ERR_ARG, "bad arguments");
+    if (!us || n <= 0) return fail(c, VV_ERR_ARG, "bad arguments");
     try {
         p.resize((size_t)n);
     } catch (const std::bad_alloc&) {
