@@ -14,9 +14,9 @@
 // first, takes a segment's samples again (in pieces of at most 64, the last
 // piece first), keeps the piece in local memory and back-propagates through it
 // in reverse: no descent is repeated.  The last quarter of a ray's records, and
-// all of them outside the unit box, are points to walk from instead (one
-// whenever 32 or more samples were composited since the last), for rays that
-// cross more segments than there are records.  The control flow (descent, step counts, early
+// all of them where the unit box's walk is not taken, are points to walk from
+// instead (one whenever 32 or more samples were composited since the last), for
+// rays that cross more segments than there are records.  The control flow (descent, step counts, early
 // termination) is that of the forward and is held fixed, as any reverse-mode
 // derivative of this shader does.
 #include "ckpt_layout.h"
@@ -517,7 +517,7 @@ __device__ __forceinline__ void backward_pixel(const RaycastParams& p, int px, i
     }
 }
 
-// The same for a volume box other than [0,1]^3: every record is walked from.
+// The same where the unit box's walk is not taken: every record is walked from.
 template <int FMT, bool F64, bool WSUM>
 __device__ __forceinline__ void backward_pixel_box(const RaycastParams& p, int px, int py, const int2* hdr,
                                                 const Ckpt* ckpt, int per_ray, const float4* dl_dcolor,

@@ -29,8 +29,9 @@ using namespace rc;
 // 7 resident CTAs (28 warps) per SM: at most 72 registers per thread.  Whole
 // draws at 4 / 5 / 6 / 7 / 8 CTAs: 2160p over the 2048^3 terrain 7.18 / 6.58 /
 // 6.38 / 6.21 / 6.12 ms, the 256^3 volume at 512x512 0.290 / 0.279 / 0.284 /
-// 0.281 / 0.282 ms, DXT5 there 0.552 / 0.553 / 0.541 / 0.537 / 0.531; lit there
-// 0.381 / 0.386 / 0.386 / 0.396 / 0.399, so lit draws take 5.
+// 0.281 / 0.282 ms, DXT5 there 0.552 / 0.553 / 0.541 / 0.537 / 0.531 (7 is
+// within 1.5 % of the best of each); lit there 0.381 / 0.386 / 0.386 / 0.396 /
+// 0.399: lit draws take 5, 1.3 % over the best.
 template <int FMT, bool COUNT, bool LIT, int RAYS>
 __global__ void __launch_bounds__(128, LIT ? 5 : 7) raycast_kernel(const __grid_constant__ RaycastParams p) {
     int px, py;

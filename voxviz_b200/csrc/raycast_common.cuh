@@ -4,9 +4,13 @@
 // Floating point: every translation unit that includes this header is
 // compiled with -fmad=false -prec-div=true -prec-sqrt=true and without
 // fast-math, so each +,-,*,/ and sqrt below is one IEEE binary32 operation in
-// the written order; the only fused operation is the explicit fmaf() of
-// lerpf().  The host oracle performs the same sequence, which makes descent
-// decisions, step counts, LOD choices and node-usage lists bit-identical.
+// the written order.  Fused operations are written as such: the linear
+// interpolations of the filter (fma2 in lerp4 and lerp_x, as the oracle's
+// lerp is fused); the corrections of fixed_div and markstein_div
+// (fixed_div.h), whose quotients equal the IEEE division; and the bounds of
+// brick_empty, which only pick samples that are zero.  The host oracle performs
+// the same sequence, which makes descent decisions, step counts, LOD choices and
+// node-usage lists bit-identical.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -40,7 +44,6 @@ __device__ __forceinline__ F3 normalize3(F3 v) {
     float r = 1.0f / sqrtf(dot3(v, v));
     return muls(v, r);
 }
-__device__ __forceinline__ float lerpf(float a, float b, float t) { return fmaf(t, b - a, a); }
 
 __device__ __forceinline__ void set_status(int* status, int code) {
     if (status) atomicCAS(status, 0, code);
@@ -62,21 +65,14 @@ template <int FMT>
 struct Texel;
 // Byte k of v as a float, exactly: the bit pattern 0x4B0000bb is 2^23 + b.
 // (A byte-select and an add instead of an integer-to-float conversion, which
-// runs at a quarter of the add rate.)
+// runs at a quarter of the add rate.)  Selectors: result bytes (low to high) =
+// byte k of v, 0, 0, 0x4B.
 __device__ __forceinline__ float byte_as_float(uint32_t v, uint32_t sel) {
     return __uint_as_float(__byte_perm(v, 0x4B000000u, sel)) - 8388608.0f;
 }
 template <>
 struct Texel<VV_FMT_RGBA8> {
     static constexpr float kScale = 1.0f / 255.0f;
-    __device__ __forceinline__ static float4 unpack(uint32_t v) {
-        // selectors: result bytes (low to high) = byte k of v, 0, 0, 0x4B
-        return make_float4(byte_as_float(v, 0x7440u), byte_as_float(v, 0x7441u), byte_as_float(v, 0x7442u),
-                           byte_as_float(v, 0x7443u));
-    }
-    __device__ __forceinline__ static float4 load(const void* pool, uint32_t i) {
-        return unpack(__ldg((const uint32_t*)pool + i));
-    }
 };
 template <>
 struct Texel<VV_FMT_FP16> {
@@ -169,7 +165,7 @@ struct Pair4 {
     unsigned long long xy, zw;
 };
 __device__ __forceinline__ Pair4 pair4(float4 v) { return Pair4{pack2(v.x, v.y), pack2(v.z, v.w)}; }
-// lerpf of every channel, tt = (t, t)
+// fmaf(t, b - a, a) of every channel, tt = (t, t)
 __device__ __forceinline__ Pair4 lerp4(Pair4 a, Pair4 b, unsigned long long tt) {
     return Pair4{fma2(tt, sub2(b.xy, a.xy), a.xy), fma2(tt, sub2(b.zw, a.zw), a.zw)};
 }
@@ -1441,7 +1437,13 @@ __device__ __forceinline__ void render_pixel(const RaycastParams& p, int px, int
 // 199; 256x192: 140 / 202 / 298, 124 / 169 / 263, 140 / 212 / 273, 155 / 220 /
 // 260; 384x288: 156 / 232 / 308, 149 / 195 / 306, 189 / 278 / 335; 512x512:
 // 174 / 292 / 336, 213 / 292 / 346), until the warps are more than the
-// machine holds: the lines of rays_per_warp.
+// machine holds: the lines of rays_per_warp.  Other draws and the adjoint have
+// the first line in the same place (4 / 16 / 32 rays, lit 192x128 205 / 210 /
+// 257, 256x192 281 / 208 / 259; DXT5 228 / 230 / 282, 334 / 240 / 288; FP32 154 /
+// 171 / 203, 200 / 169 / 204; forward and adjoint of 160x120 544 / 535 / 572, of
+// two 128x128 833 / 688 / 666), the second lower: 384x288 lit 506 / 272 / 257,
+// DXT5 605 / 337 / 304, forward and adjoint 1604 / 1171 / 1069, up to a tenth
+// under the one line that all of them share.
 __host__ __device__ constexpr int warp_tile_w(int rays) { return rays == 32 ? 8 : rays == 16 ? 4 : 2; }
 __host__ __device__ constexpr int warp_tile_h(int rays) { return rays == 32 ? 4 : rays == 16 ? 4 : 2; }
 inline int rays_per_warp(long long rays) { return rays <= 24576 ? 4 : rays <= 114688 ? 16 : 32; }
