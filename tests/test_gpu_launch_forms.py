@@ -97,3 +97,37 @@ def test_odd_frames_of_an_autograd_call(size, spread):
     got = got.cpu().numpy().astype(np.float64)
     assert np.abs(ref).max() > 0
     assert (np.abs(got - ref) <= 1e-3 * np.abs(ref) + 1e-5 * mag).all()
+
+
+@pytest.mark.parametrize("form", [{}, {"f64": True}, {"warp_sum": True}, {"spread": True}])
+@pytest.mark.parametrize("boxes,size", [("ubbuu", (33, 21)), ("b" * 18, (19, 13)), ("bu" * 3, (19, 13)), ("bb", (161, 157))])
+def test_views_of_several_boxes(form, boxes, size):
+    """Unit boxes (u) and others (b) in one call: each run of a kind is a launch."""
+    sc = helpers.Scene(seed=1, depth=4, fmt="rgba8")
+    g = helpers.GpuScene(sc)
+    W, H = size
+    n, slots = len(boxes), sc.pool.shape[0]
+    us = [sc.uniforms(sc.view(3 + v, W, H)) for v in range(n)]
+    for u, b in zip(us, boxes):
+        if b == "b":
+            u.vol_extent_max[2] = 0.75
+    ck = torch.zeros((n, vv.Context.ckpt_bytes(W, H, 4)), dtype=torch.uint8, device="cuda")
+    color = torch.zeros((n, H, W, 4), device="cuda")
+    g.ctx.forward_ckpt_views(us, color.data_ptr(), ck.data_ptr(), 4)
+    dl = np.random.default_rng(n).standard_normal((n, H, W, 4)).astype(np.float32)
+    dl_t = torch.from_numpy(dl).cuda()
+    grad = torch.zeros((slots, 1000, 4), dtype=torch.float64 if form.get("f64") else torch.float32, device="cuda")
+    g.ctx.backward_views(us, dl_t.data_ptr(), ck.data_ptr(), 4, grad.data_ptr(), **form)
+    g.ctx.synchronize()
+    status = g.ctx.device_status(clear=True)  # (rays of a box may end at the iteration bound, as the oracle's do)
+    mag, ref = np.zeros((slots, 1000, 4)), np.zeros((slots, 1000, 4))
+    want = 0
+    for v in range(n):
+        frame = g.render(us[v], passes=vv.VV_PASS_RAYCAST)
+        want = want or frame["status"]
+        assert np.array_equal(color[v].cpu().numpy(), frame["color"])
+        go.backward(us[v], sc.oracle_scene(), dl[v], grad=ref, grad_abs=mag)
+    assert status == want
+    got = grad.cpu().numpy().astype(np.float64)
+    assert np.abs(ref).max() > 0
+    assert (np.abs(got - ref) <= 1e-3 * np.abs(ref) + 1e-5 * mag).all()

@@ -595,18 +595,24 @@ __global__ void __launch_bounds__(128, 4)
                                    PathSlots{&path[0][threadIdx.x], 128, nullptr});
 }
 
-// A view of another box, in a kernel of its own: as a function that the kernel
-// above called for such a view it ran a lane at a time.  One backward of the
-// 1024^3 terrain in a box of three quarters at 960x540 / the 512^3 one at
-// 1920x1080 / the 256^3 one at 256x256: 6.27 / 6.20 / 1.28 ms as a function,
-// 1.58 / 3.72 / 0.49 ms here (6 CTAs per SM; 1.59 / 3.81 / 0.49 at 5).
-template <int FMT, bool F64, bool WSUM>
+// The views of other boxes, in a kernel of its own: as a function that the
+// kernel above called for such a view it ran a lane at a time.  One backward of
+// the 1024^3 terrain in a box of three quarters at 960x540 / the 512^3 one at
+// 1920x1080 / the 256^3 one at 256x256: 6.27 / 6.20 / 1.28 ms as a function, 1.61
+// / 3.88 / 0.53 ms here (6 CTAs per SM, 80 registers; 5 the same).  17 views of
+// 96x96 in one launch of 16 and one: fit step 2.34 ms, a launch each 13.0.
+template <int FMT, bool F64, bool WSUM, int VIEWS>
 __global__ void __launch_bounds__(128, 6)
-    backward_box_kernel(const __grid_constant__ RaycastParams p, const char* ckpts, size_t hdr_size, int per_ray,
-                        const float4* dl, const __grid_constant__ GradTarget gt) {
+    backward_box_kernel(const __grid_constant__ DiffViews<VIEWS> dv, const char* ckpts, size_t stride, size_t hdr_size,
+                        int per_ray, const float4* dl, const __grid_constant__ GradTarget gt, int rays) {
+    const RaycastParams& p = dv.p[VIEWS > 1 ? blockIdx.z : 0];
+    const char* ck = ckpts + (VIEWS > 1 ? blockIdx.z * stride : 0);
+    const float4* dl_dcolor = dl + (VIEWS > 1 ? (size_t)blockIdx.z * p.u.width * p.u.height : 0);
     int px, py;
-    warp_pixel<32>(px, py);
-    backward_pixel_box<FMT, F64, WSUM>(p, px, py, (const int2*)ckpts, (const Ckpt*)(ckpts + hdr_size), per_ray, dl, gt);
+    if (rays == 4) warp_pixel<4>(px, py);
+    else if (rays == 16) warp_pixel<16>(px, py);
+    else warp_pixel<32>(px, py);
+    backward_pixel_box<FMT, F64, WSUM>(p, px, py, (const int2*)ck, (const Ckpt*)(ck + hdr_size), per_ray, dl_dcolor, gt);
 }
 
 // grad[e] += copy_k[e] for the extra copies k of the rows in use (all rows
@@ -695,12 +701,17 @@ cudaError_t backward_views(const RaycastParams* p, int n, const char* ckpt, size
     return cudaGetLastError();
 }
 
-template <int FMT, bool F64, bool WSUM>
-cudaError_t backward_view(const RaycastParams* p, const char* ckpt, size_t stride, int per_ray, const float4* dl,
-                          const GradTarget& gt, cudaStream_t s) {
-    if (takes_unit_walk(*p)) return backward_views<FMT, F64, WSUM, 1>(p, 1, ckpt, stride, per_ray, dl, gt, s);
+// Views that take the unit box's walk, or views that do not.
+template <int FMT, bool F64, bool WSUM, int VIEWS>
+cudaError_t backward_run(const RaycastParams* p, int n, const char* ckpt, size_t stride, int per_ray, const float4* dl,
+                         const GradTarget& gt, cudaStream_t s) {
+    if (takes_unit_walk(*p)) return backward_views<FMT, F64, WSUM, VIEWS>(p, n, ckpt, stride, per_ray, dl, gt, s);
     const int W = p->u.width, H = p->u.height;
-    backward_box_kernel<FMT, F64, WSUM><<<warp_grid(32, W, H), 128, 0, s>>>(*p, ckpt, ckpt_header_bytes(W, H), per_ray, dl, gt);
+    DiffViews<VIEWS> dv;
+    for (int v = 0; v < n; ++v) dv.p[v] = p[v];
+    const int rays = F64 || WSUM ? 32 : rays_per_warp((long long)n * W * H);
+    backward_box_kernel<FMT, F64, WSUM, VIEWS><<<warp_grid(rays, W, H, n), 128, 0, s>>>(
+        dv, ckpt, stride, ckpt_header_bytes(W, H), per_ray, dl, gt, rays);
     return cudaGetLastError();
 }
 
@@ -708,24 +719,17 @@ template <int FMT>
 cudaError_t backward_form(const RaycastParams* p, int n, const char* ckpt, size_t stride, int per_ray, const float4* dl,
                           const GradTarget& gt, cudaStream_t s) {
     const size_t npix = (size_t)p->u.width * p->u.height;
+    const int most = gt.f64 || gt.warp_sum ? 1 : kMaxDiffViews;
     cudaError_t e = cudaSuccess;
-    for (int v = 0; v < n && e == cudaSuccess; v += kMaxDiffViews) {
-        const int m = n - v < kMaxDiffViews ? n - v : kMaxDiffViews;
-        bool unit = true;
-        for (int i = v; i < v + m; ++i) unit = unit && takes_unit_walk(p[i]);
-        if (m > 1 && unit && !gt.f64 && !gt.warp_sum) {
-            e = backward_views<FMT, false, false, kMaxDiffViews>(p + v, m, ckpt + (size_t)v * stride, stride, per_ray,
-                                                                 dl + (size_t)v * npix, gt, s);
-            continue;
-        }
-        for (int i = v; i < v + m && e == cudaSuccess; ++i) {
-            const char* ck = ckpt + (size_t)i * stride;
-            const float4* d = dl + (size_t)i * npix;
-            if (gt.f64 && gt.warp_sum) e = backward_view<FMT, true, true>(p + i, ck, stride, per_ray, d, gt, s);
-            else if (gt.f64) e = backward_view<FMT, true, false>(p + i, ck, stride, per_ray, d, gt, s);
-            else if (gt.warp_sum) e = backward_view<FMT, false, true>(p + i, ck, stride, per_ray, d, gt, s);
-            else e = backward_view<FMT, false, false>(p + i, ck, stride, per_ray, d, gt, s);
-        }
+    for (int v = 0, m; v < n && e == cudaSuccess; v += m) {
+        for (m = 1; m < most && v + m < n && takes_unit_walk(p[v + m]) == takes_unit_walk(p[v]);) ++m;
+        const char* ck = ckpt + (size_t)v * stride;
+        const float4* d = dl + (size_t)v * npix;
+        if (m > 1) e = backward_run<FMT, false, false, kMaxDiffViews>(p + v, m, ck, stride, per_ray, d, gt, s);
+        else if (gt.f64 && gt.warp_sum) e = backward_run<FMT, true, true, 1>(p + v, 1, ck, stride, per_ray, d, gt, s);
+        else if (gt.f64) e = backward_run<FMT, true, false, 1>(p + v, 1, ck, stride, per_ray, d, gt, s);
+        else if (gt.warp_sum) e = backward_run<FMT, false, true, 1>(p + v, 1, ck, stride, per_ray, d, gt, s);
+        else e = backward_run<FMT, false, false, 1>(p + v, 1, ck, stride, per_ray, d, gt, s);
     }
     return e;
 }
